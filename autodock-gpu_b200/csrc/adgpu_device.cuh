@@ -56,21 +56,37 @@ struct __align__(16) PairRec {
 
 // Two pairs of the AD4 force field (exponents m = 12 and n = 6 or 10), the
 // ones one thread takes in one step of the pair loop: pair A of an aligned
-// group of 32 pairs (one warp instruction) and pair B of the next group,
-// 64 bytes in four quads whose fields interleave A and B, so packed FP32x2
-// instructions take both pairs' operands straight from the loaded registers:
+// group of 32 pairs (one warp instruction) and pair B of the next group, in
+// three quads whose fields interleave A and B, so packed FP32x2 instructions
+// take both pairs' operands straight from the loaded registers, and one word
+// (coupled records) or two that name the atoms:
 //   q0 = (AC_A, AC_B, b6_A, b6_B)     VWpars_AC; VWpars_BD of a 12-6 pair, else 0
 //   q1 = (b10_A, b10_B, reqm_A, reqm_B)  VWpars_BD of a 12-10 pair, else 0; reqm_AB
 //   q2 = (ds_A, ds_B, qq_A, qq_B)     coeff_desolv*((S1+qasp|q1|)V2 + (S2+qasp|q2|)V1); coeff_elec*q1*q2
-//   q3 = (G_A, G_B, ij_A, ij_B)       G of a CG-G0 pair, else 0; atom1 | atom2 << 8
+//   coupled:   shared atom | A's other atom << 10 | B's other atom << 20 | cg_A << 30 | cg_B << 31
+//   otherwise: A1 | A2 << 10 | cg_A << 30, and B1 | B2 << 10 | cg_B << 30 (cg: a CG-G0 pair)
 // With BD in b6 or b10 by the pair's n (the other 0) the vdW/H-bond energy is
 // AC/sd^12 - b6/sd^6 - b10/sd^10 with no select.  The 32 records of a group
-// pair are stored quad by quad (quad j of record r at float4 index
-// (r/32)*128 + j*32 + r%32), so a warp's load of one quad reads 512
-// contiguous bytes.  Padding entries (lists are whole group pairs) have every
-// coefficient 0 and both atoms the same: they add exactly 0 to energies and
-// forces.
-__host__ __device__ inline uint32_t pair2_quad(uint32_t rec, uint32_t j) { return (rec / 32u) * 128u + j * 32u + rec % 32u; }
+// pair are one block, stored quad by quad and then word by word (quad j of
+// record r at float4 index (r/32)*B + j*32 + r%32), so a warp's load of one
+// quad reads 512 contiguous bytes.  A warp's step loads 52 bytes a record, 13
+// wavefronts of the L1 data pipe that bounds the pair loop (with G and both
+// atoms' words in a fourth quad it was 16).  Padding entries (lists are whole
+// group pairs) have every coefficient 0 and both atoms the same: they add
+// exactly 0 to energies and forces.
+constexpr uint32_t kPairAtomBits = 10, kPairAtomMask = (1u << kPairAtomBits) - 1u;
+constexpr float kGBond = 50.0f;      // G of a CG-G0 pair, common/defines.h:108
+// float4s of a block of 32 records
+__host__ __device__ constexpr uint32_t pair2_block(bool coupled) { return coupled ? 104u : 112u; }
+__host__ __device__ inline uint32_t pair2_quad(bool coupled, uint32_t rec, uint32_t j)
+{
+	return (rec / 32u) * pair2_block(coupled) + j * 32u + rec % 32u;
+}
+// word h (0; 1 of an uncoupled record) of record rec
+__host__ __device__ inline uint32_t* pair2_word(bool coupled, float4* Q, uint32_t rec, uint32_t h)
+{
+	return reinterpret_cast<uint32_t*>(Q + (rec / 32u) * pair2_block(coupled) + 96u) + h * 32u + rec % 32u;
+}
 
 // Slot (record, half) of the s-th pair of the ordered list of AD4 pairs:
 // group s/32 is half (s/32) % 2 of records (s/64)*32 .. +31, lane s % 32.
@@ -82,26 +98,26 @@ __host__ __device__ inline void pair2_slot(uint32_t s, uint32_t* rec, uint32_t* 
 // Records for n ordered AD4 pairs (whole groups of 64 pairs, padded).
 __host__ __device__ inline uint32_t pair2_records(uint32_t n) { return (n + 63u) / 64u * 32u; }
 
-// Writes one pair into half h of record rec (quads Q).
-__host__ __device__ inline void pair2_set(float4* Q, uint32_t rec, uint32_t h, float ac, float b6, float b10, float reqm,
-                                          float ds, float qq, float vb, uint32_t ij)
+// Writes the coefficients of one pair into half h of record rec (quads Q).
+__host__ __device__ inline void pair2_set(bool coupled, float4* Q, uint32_t rec, uint32_t h, float ac, float b6, float b10,
+                                          float reqm, float ds, float qq)
 {
-	float* q0 = reinterpret_cast<float*>(Q + pair2_quad(rec, 0));
-	float* q1 = reinterpret_cast<float*>(Q + pair2_quad(rec, 1));
-	float* q2 = reinterpret_cast<float*>(Q + pair2_quad(rec, 2));
-	float* q3 = reinterpret_cast<float*>(Q + pair2_quad(rec, 3));
+	float* q0 = reinterpret_cast<float*>(Q + pair2_quad(coupled, rec, 0));
+	float* q1 = reinterpret_cast<float*>(Q + pair2_quad(coupled, rec, 1));
+	float* q2 = reinterpret_cast<float*>(Q + pair2_quad(coupled, rec, 2));
 	q0[h] = ac; q0[2 + h] = b6;
 	q1[h] = b10; q1[2 + h] = reqm;
 	q2[h] = ds; q2[2 + h] = qq;
-	q3[h] = vb; reinterpret_cast<uint32_t*>(q3)[2 + h] = ij;
 }
 // A padding record (both halves) for lane position rec % 32 of an N-atom
 // ligand: the atoms are spread so that padded lanes do not all hit one
 // shared-memory bank.
-__host__ __device__ inline void pair2_pad(float4* Q, uint32_t rec, uint32_t N)
+__host__ __device__ inline void pair2_pad(bool coupled, float4* Q, uint32_t rec, uint32_t N)
 {
 	const uint32_t a = (rec % 32u) % N;
-	for (uint32_t h = 0; h < 2; h++) pair2_set(Q, rec, h, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f, a | (a << 8));
+	for (uint32_t h = 0; h < 2; h++) pair2_set(coupled, Q, rec, h, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f);
+	*pair2_word(coupled, Q, rec, 0) = coupled ? a | (a << kPairAtomBits) | (a << (2 * kPairAtomBits)) : a | (a << kPairAtomBits);
+	if (!coupled) *pair2_word(coupled, Q, rec, 1) = a | (a << kPairAtomBits);
 }
 
 // Stored position of element p of a list of n (torsion items; pairs in the
@@ -126,6 +142,7 @@ struct LigDev {
 	int natoms, nlig, ngenes, ntors, npairs, ntoritems;
 	int npairs2, ngpairs;
 	int coupled;                 // 1: the two pairs of every record share their first atom
+	int cgg0;                    // 1: some AD4 pair is a CG-G0 pair
 	int map_e;                   // index of the e map in the cell record (0)
 	// grid
 	int gx, gy, gz;              // grid points per axis
@@ -305,14 +322,16 @@ struct Group {
 
 // ---- per-pose shared-memory scratch -------------------------------------------------
 // Layout (natoms rounded up to a multiple of 4):
-//   tq [ntors] float4; xyz [N] float4 (x, y, z, 0); f3 [3N] int; gg [64] int
-// An atom's coordinates are one 16-byte load, so a pair reads both its atoms
-// with two shared-memory loads.  Its fixed-point force is f3[3a .. 3a+2]:
-// one address per atom for the three components, and since 3 is odd, atoms
-// whose indices differ mod 32 fall in different banks, as in three separate
-// arrays.
+//   tq [ntors] float4; gsc; xyz [3N] float; f3 [3N] int; gg [64] int
+// An atom's coordinates are xyz[3a .. 3a+2] and its fixed-point force is
+// f3[3a .. 3a+2]: one address per atom for the three components, and since 3
+// is odd, atoms whose indices differ mod 32 fall in different banks, as in
+// three separate arrays.  (As one 16-byte load per atom, coordinates took
+// four wavefronts at least and 8.5 on average in the pair loop, since only
+// eight lanes go in one and their atoms collide mod 8; three 4-byte loads
+// take 5.8 together.)
 struct PoseSmem {
-	float4* xyz;
+	float* xyz;
 	int* f3;
 	float4* tq;
 	float2* gsc;       // sin/cos of theta, phi and half the rotation angle
@@ -322,7 +341,7 @@ struct PoseSmem {
 __host__ __device__ inline int pose_smem_bytes(int natoms, int ntors)
 {
 	int n4 = (natoms + 3) & ~3;
-	return (7 * n4) * 4 + ntors * 16 + 32 + 64 * 4;
+	return (6 * n4) * 4 + ntors * 16 + 32 + 64 * 4;
 }
 
 __device__ __forceinline__ PoseSmem carve_pose(char* base, int natoms, int ntors)
@@ -334,8 +353,8 @@ __device__ __forceinline__ PoseSmem carve_pose(char* base, int natoms, int ntors
 	f += ntors * 4;
 	s.gsc = reinterpret_cast<float2*>(f);
 	f += 8;
-	s.xyz = reinterpret_cast<float4*>(f);         // still 16-byte aligned
-	f += 4 * n4;
+	s.xyz = f;                                    // still 16-byte aligned
+	f += 3 * n4;
 	s.f3 = reinterpret_cast<int*>(f);
 	s.gg = s.f3 + 3 * n4;
 	return s;
@@ -396,6 +415,9 @@ static __device__ __noinline__ float pow_int(float b, int e)
 	return r;
 }
 
+// An atom's coordinates in shared memory.
+__device__ __forceinline__ float3 ld3(const float* p) { return make_float3(p[0], p[1], p[2]); }
+
 // The fixed-point force of one pair (components already scaled by 1024):
 // -q on the first atom, +q on the second (f3: three ints per atom).
 __device__ __forceinline__ void pair_force(int* f3, uint32_t i, uint32_t j, float gx, float gy, float gz)
@@ -443,8 +465,9 @@ __device__ __forceinline__ void couple_force(unsigned* f3, uint32_t c, uint32_t 
 // TERMS (energy only): also adds this thread's vdW/H-bond, electrostatic,
 // desolvation and CG-G0 sums to tsum[0..3].
 // With COUPLED (the host's tables, L.coupled) the two pairs of a record share
-// their first atom: one position load and one set of atomics for it.
-template <int TPP, bool GRAD, bool TERMS, bool COUPLED>
+// their first atom: one position load and one set of atomics for it.  CGG0:
+// the ligand has CG-G0 pairs (flexible rings).
+template <int TPP, bool GRAD, bool TERMS, bool COUPLED, bool CGG0>
 __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, int rank, float* tsum)
 {
 	// loop invariants read once: when L lives in shared memory (the engine's
@@ -454,19 +477,23 @@ __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, i
 	const float inv_emd = __fdividef(1.0f, emd);
 	const int nrec = L.npairs2;
 	const float spacing = L.spacing, inv_spacing = L.inv_spacing;
-	const float4* const xyz = S.xyz;
+	const float* const xyz = S.xyz;
 	int* const f3 = S.f3;
 	float2 esum = f2s(0.0f);
 	float2 t_vdw = f2s(0.0f), t_el = f2s(0.0f), t_ds = f2s(0.0f), t_cg = f2s(0.0f);
-	// record d = rank + TPP*i: quads at pair2_quad(d, j); the pointer steps
-	// TPP/32 blocks of 128 quads per iteration
-	const float4* pr = L.pairs2 + (rank / 32) * 128 + (rank % 32);
-	for (int d = rank; d < nrec; d += TPP, pr += (TPP / 32) * 128) {
-		const float4 q0 = __ldg(pr), q1 = __ldg(pr + 32), q2 = __ldg(pr + 64), q3 = __ldg(pr + 96);
-		const uint32_t ija = __float_as_uint(q3.z), ijb = __float_as_uint(q3.w);
-		const uint32_t a1 = ija & 0xFFu, a2 = ija >> 8, b1 = COUPLED ? a1 : (ijb & 0xFFu), b2 = ijb >> 8;
-		const float4 pa1 = xyz[a1], pa2 = xyz[a2], pb2 = xyz[b2];
-		const float4 pb1 = COUPLED ? pa1 : xyz[b1];
+	// record d = rank + TPP*i: quads at pair2_quad(d, j), words behind the
+	// block's quads; the pointers step TPP/32 blocks per iteration
+	constexpr int kBlock = (int)pair2_block(COUPLED);
+	const float4* pr = L.pairs2 + (rank / 32) * kBlock + (rank % 32);
+	const uint32_t* pw = reinterpret_cast<const uint32_t*>(L.pairs2 + (rank / 32) * kBlock + 96) + (rank % 32);
+	for (int d = rank; d < nrec; d += TPP, pr += (TPP / 32) * kBlock, pw += (TPP / 32) * kBlock * 4) {
+		const uint32_t wa = __ldg(pw), wb = COUPLED ? 0u : __ldg(pw + 32);
+		const float4 q0 = __ldg(pr), q1 = __ldg(pr + 32), q2 = __ldg(pr + 64);
+		const uint32_t a1 = wa & kPairAtomMask, a2 = (wa >> kPairAtomBits) & kPairAtomMask;
+		const uint32_t b1 = COUPLED ? a1 : (wb & kPairAtomMask);
+		const uint32_t b2 = (COUPLED ? wa >> (2 * kPairAtomBits) : wb >> kPairAtomBits) & kPairAtomMask;
+		const float3 pa1 = ld3(xyz + 3 * a1), pa2 = ld3(xyz + 3 * a2), pb2 = ld3(xyz + 3 * b2);
+		const float3 pb1 = COUPLED ? pa1 : ld3(xyz + 3 * b1);
 		const float2 sx = f2(pa1.x - pa2.x, pb1.x - pb2.x);
 		const float2 sy = f2(pa1.y - pa2.y, pb1.y - pb2.y);
 		const float2 sz = f2(pa1.z - pa2.z, pb1.z - pb2.z);
@@ -474,10 +501,12 @@ __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, i
 		// coincident atoms (d2g = 0) get r = 0 from a finite reciprocal
 		const float2 inv_dist = f2(rsqrtf(fmaxf(d2g.x, 1e-30f)), rsqrtf(fmaxf(d2g.y, 1e-30f)));
 		const float2 r = f2mul(f2mul(d2g, inv_dist), f2s(spacing));
-		const float2 vb = f2(q3.x, q3.y);             // G for CG-G0 pairs, else 0
-		float2 e = f2mul(vb, r);
-		float2 pg = vb;
-		if constexpr (TERMS) t_cg = f2add(t_cg, e);
+		float2 e = f2s(0.0f), pg = f2s(0.0f);
+		if constexpr (CGG0) {
+			pg = f2((wa >> 30) & 1u ? kGBond : 0.0f, (COUPLED ? wa >> 31 : (wb >> 30) & 1u) ? kGBond : 0.0f);
+			e = f2mul(pg, r);
+			if constexpr (TERMS) t_cg = f2add(t_cg, e);
+		}
 		// vdW / H-bond, cut-off 8 A
 		{
 			const float2 lo = f2add(r, f2s(-hs)), hi = f2add(r, f2s(hs));
@@ -551,8 +580,9 @@ __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, i
 template <int TPP, bool GRAD, bool TERMS = false>
 __device__ __forceinline__ float pair_terms(const LigDev& L, const PoseSmem& S, int rank, float* tsum = nullptr)
 {
-	return L.coupled ? pair_loop<TPP, GRAD, TERMS, true>(L, S, rank, tsum)
-	                 : pair_loop<TPP, GRAD, TERMS, false>(L, S, rank, tsum);
+	if (!L.coupled) return pair_loop<TPP, GRAD, TERMS, false, true>(L, S, rank, tsum);
+	return L.cgg0 ? pair_loop<TPP, GRAD, TERMS, true, true>(L, S, rank, tsum)
+	              : pair_loop<TPP, GRAD, TERMS, true, false>(L, S, rank, tsum);
 }
 
 // Pairs with other exponents than 12-6 / 12-10 (modified pair potentials;
@@ -567,7 +597,7 @@ __device__ __forceinline__ float pair_terms_generic(const LigDev& L, const PoseS
 		const PairRec P = L.gpairs[p];
 		const uint32_t a1 = P.ij & 0xFFu, a2 = (P.ij >> 8) & 0xFFu;
 		const int m = (int)((P.ij >> 16) & 0xFFu), n = (int)(P.ij >> 24);
-		const float4 p1 = S.xyz[a1], p2 = S.xyz[a2];
+		const float3 p1 = ld3(S.xyz + 3 * a1), p2 = ld3(S.xyz + 3 * a2);
 		const float sx = p1.x - p2.x, sy = p1.y - p2.y, sz = p1.z - p2.z;
 		const float d2g = sx * sx + sy * sy + sz * sz;
 		const float inv_dist = rsqrtf(fmaxf(d2g, 1e-30f));
@@ -667,7 +697,7 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 			p = qrot(p, gr.q);
 			p.x += gr.mv.x; p.y += gr.mv.y; p.z += gr.mv.z;
 		}
-		S.xyz[a] = make_float4(p.x, p.y, p.z, 0.0f);
+		S.xyz[3 * a] = p.x; S.xyz[3 * a + 1] = p.y; S.xyz[3 * a + 2] = p.z;
 
 		// 3. intermolecular: trilinear interpolation of the type, e and d maps
 		//    (cuda/calcMergeEneGra.cu:195-413)
@@ -760,7 +790,7 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 	const float spacing = L.spacing;
 	float red[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, e_acc};
 	for (int a = rank; a < nlig; a += TPP) {
-		const float4 pa = S.xyz[a];
+		const float3 pa = ld3(S.xyz + 3 * a);
 		float3 r = make_float3((pa.x - gr.mv.x) * spacing, (pa.y - gr.mv.y) * spacing, (pa.z - gr.mv.z) * spacing);
 		const int* fa = S.f3 + 3 * a;
 		float3 f = make_float3(kOneOverTermScale * (float)fa[0], kOneOverTermScale * (float)fa[1], kOneOverTermScale * (float)fa[2]);
@@ -816,7 +846,7 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 		uint32_t item = tor_items[it];
 		int k = item >> 8, la = item & 0xFF;
 		int2 ends = tors_ends[k];
-		const float4 e0 = S.xyz[ends.x], e1 = S.xyz[ends.y], pl = S.xyz[la];
+		const float3 e0 = ld3(S.xyz + 3 * ends.x), e1 = ld3(S.xyz + 3 * ends.y), pl = ld3(S.xyz + 3 * la);
 		float rx = e0.x, ry = e0.y, rz = e0.z;
 		float ux = e1.x - rx, uy = e1.y - ry, uz = e1.z - rz;
 		float l = rnorm3df(ux, uy, uz);

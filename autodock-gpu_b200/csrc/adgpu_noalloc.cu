@@ -54,7 +54,7 @@ NoAllocLayout layout_for(const adgpu_dockpars& dp)
 	l.mv = o; o = up16(o + (NT + 1) * 16);
 	l.ends = o; o = up16(o + (NT + 1) * 8);
 	l.items = o; o = up16(o + N * (NT + 1) * 4);
-	// AD4 pairs take pair2_records(Qs) * 64 <= 32 * Qs + 2048 bytes and the
+	// AD4 pairs take pair2_records(Qs) * 56 <= 32 * Qs + 2048 bytes and the
 	// others 32 * Qg, so this holds any split of the Q pairs
 	l.pairs = o; l.pairs_bytes = (size_t)pair2_records((uint32_t)Q) * 64 + 32 * 64;
 	o = up16(o + l.pairs_bytes);
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(256) noalloc_repack_kernel(adgpu_gpudata d, Li
 	const uint32_t nrec = pair2_records((uint32_t)Qs);
 	float4* pr2 = reinterpret_cast<float4*>(base + lay.pairs);
 	PairRec* gpr = reinterpret_cast<PairRec*>(base + lay.pairs + lay.pairs_bytes - (size_t)Qg * sizeof(PairRec));
-	for (uint32_t r = threadIdx.x; r < nrec; r += blockDim.x) pair2_pad(pr2, r, (uint32_t)N);
+	for (uint32_t r = threadIdx.x; r < nrec; r += blockDim.x) pair2_pad(false, pr2, r, (uint32_t)N);
 	__syncthreads();
 	int gi = s_gen[threadIdx.x];
 	for (int p = p0; p < p1; p++) {
@@ -205,12 +205,12 @@ __global__ void __launch_bounds__(256) noalloc_repack_kernel(adgpu_gpudata d, Li
 		const float dsp = __fadd_rn(__fmul_rn(__fadd_rn(kin->dspars_S_const[t1], __fmul_rn(dp.qasp, fabsf(q1))), kin->dspars_V_const[t2]),
 		                            __fmul_rn(__fadd_rn(kin->dspars_S_const[t2], __fmul_rn(dp.qasp, fabsf(q2))), kin->dspars_V_const[t1]));
 		const float qq = __fmul_rn(__fmul_rn(dp.coeff_elec, q1), q2);
-		const float vb = cgg0 ? 50.0f : 0.0f;
+		const float vb = cgg0 ? kGBond : 0.0f;
 		if (is_ad4(exps)) {
 			uint32_t rec, h;
 			pair2_slot(interleave_pos((uint32_t)(p - gi), (uint32_t)Qs), &rec, &h);
-			pair2_set(pr2, rec, h, ac, n == 6 ? bd : 0.0f, n == 10 ? bd : 0.0f, reqm, __fmul_rn(dp.coeff_desolv, dsp), qq,
-			          vb, a1 | (a2 << 8));
+			pair2_set(false, pr2, rec, h, ac, n == 6 ? bd : 0.0f, n == 10 ? bd : 0.0f, reqm, __fmul_rn(dp.coeff_desolv, dsp), qq);
+			*pair2_word(false, pr2, rec, h) = a1 | (a2 << kPairAtomBits) | (cgg0 ? 1u << 30 : 0u);
 		} else {
 			PairRec r;
 			r.ac = ac; r.bd = bd; r.reqm = reqm; r.dsolv_pref = dsp; r.qq = qq; r.vbond = vb;

@@ -206,7 +206,7 @@ adgpu_status pack_ligand(const adgpu_dockpars& dp, const adgpu_kc_interintra& ii
 	couple_pairs(std_pairs.data(), Qs, N, couples);
 	out.npairs2 = (int)(couples.size() + 31) / 32 * 32;
 	out.ngpairs = Qg;
-	out.off_pairs2 = o; o = align_up(o + (size_t)std::max(out.npairs2, 1) * 64, 16);
+	out.off_pairs2 = o; o = align_up(o + (size_t)(out.npairs2 / 32) * pair2_block(true) * 16, 16);
 	out.off_gpairs = o; o = align_up(o + (size_t)std::max(Qg, 1) * sizeof(PairRec), 16);
 	out.off_f3_bias = o; o = align_up(o + (size_t)N * 4, 16);
 	out.blob.assign(o, 0);
@@ -257,18 +257,20 @@ adgpu_status pack_ligand(const adgpu_dockpars& dp, const adgpu_kc_interintra& ii
 		dsolv_pref = (kin.dspars_S_const[t1] + dp.qasp * std::fabs(q1)) * kin.dspars_V_const[t2] +
 		             (kin.dspars_S_const[t2] + dp.qasp * std::fabs(q2)) * kin.dspars_V_const[t1];
 		qq = dp.coeff_elec * q1 * q2;
-		vbond = cgg0 ? 50.0f : 0.0f;
+		vbond = cgg0 ? kGBond : 0.0f;
 	};
 	float4* pr2 = reinterpret_cast<float4*>(B + out.off_pairs2);
-	for (int r = 0; r < out.npairs2; r++) pair2_pad(pr2, (uint32_t)r, (uint32_t)N);
+	for (int r = 0; r < out.npairs2; r++) pair2_pad(true, pr2, (uint32_t)r, (uint32_t)N);
 	std::vector<uint32_t> slot;
 	order_couples(std_pairs.data(), couples, slot);
 	for (size_t k = 0; k < couples.size(); k++) {
 		const Couple& cp = couples[k];
+		uint32_t word = cp.c;
 		for (uint32_t h = 0; h < 2; h++) {
 			const int q = h ? cp.b : cp.a;                 // index into the AD4 list
 			if (q < 0) {
-				pair2_set(pr2, slot[k], h, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f, cp.c | (cp.c << 8));
+				pair2_set(true, pr2, slot[k], h, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f);
+				word |= cp.c << ((1 + h) * kPairAtomBits);
 				continue;
 			}
 			const int p = std_idx[q];
@@ -276,22 +278,21 @@ adgpu_status pack_ligand(const adgpu_dockpars& dp, const adgpu_kc_interintra& ii
 			const uint32_t n = kin.VWpars_exp_const[ii.atom_types_const[a1] * (uint32_t)nat + ii.atom_types_const[a2]] & 0xFF;
 			float ac, bd, reqm, dsp, qq, vb;
 			fields(p, ac, bd, reqm, dsp, qq, vb);
-			pair2_set(pr2, slot[k], h, ac, n == 6 ? bd : 0.0f, n == 10 ? bd : 0.0f, reqm, dp.coeff_desolv * dsp, qq, vb,
-			          cp.c | (partner(std_pairs.data(), q, cp.c) << 8));
+			pair2_set(true, pr2, slot[k], h, ac, n == 6 ? bd : 0.0f, n == 10 ? bd : 0.0f, reqm, dp.coeff_desolv * dsp, qq);
+			word |= partner(std_pairs.data(), q, cp.c) << ((1 + h) * kPairAtomBits);
+			if (vb != 0.0f) { word |= 1u << (30 + h); out.cgg0 = 1; }
 		}
+		*pair2_word(true, pr2, slot[k], 0) = word;
 	}
 	// couple_force adds kRoundBits (mod 2^32) for each record's second atoms
 	// and subtracts it twice for the shared atom, padding included: each atom
 	// starts at minus the sum over the records as the kernel reads them
 	std::vector<int32_t> offsets(N, 0);
 	for (int r = 0; r < out.npairs2; r++) {
-		const float4 q3 = pr2[pair2_quad((uint32_t)r, 3)];
-		uint32_t ija, ijb;
-		std::memcpy(&ija, &q3.z, 4);
-		std::memcpy(&ijb, &q3.w, 4);
-		offsets[ija & 0xFFu] -= 2;
-		offsets[ija >> 8] += 1;
-		offsets[ijb >> 8] += 1;
+		const uint32_t w = *pair2_word(true, pr2, (uint32_t)r, 0);
+		offsets[w & kPairAtomMask] -= 2;
+		offsets[(w >> kPairAtomBits) & kPairAtomMask] += 1;
+		offsets[(w >> (2 * kPairAtomBits)) & kPairAtomMask] += 1;
 	}
 	int32_t* f3b = reinterpret_cast<int32_t*>(B + out.off_f3_bias);
 	for (int a = 0; a < N; a++) {
@@ -342,6 +343,7 @@ void place_ligand(const PackedLigand& p, const void* dbase, LigDev& L)
 	L.tor_items = reinterpret_cast<const uint32_t*>(D + p.off_tor_items);
 	L.npairs2 = p.npairs2; L.ngpairs = p.ngpairs;
 	L.coupled = 1;
+	L.cgg0 = p.cgg0;
 	L.pairs2 = reinterpret_cast<const float4*>(D + p.off_pairs2);
 	L.gpairs = reinterpret_cast<const PairRec*>(D + p.off_gpairs);
 	L.f3_bias = reinterpret_cast<const int*>(D + p.off_f3_bias);
