@@ -38,16 +38,25 @@ struct PostDev {
 	int rmsd_atoms, symmetry, rescore_all;
 	int cells;                             // grid layout: 0 reference (4 floats per point per map), 1 cell records
 	const float* grid;
+	int flex_or_cg;                        // some pair adds to interflexE: ligand-flexres or CG-G0
 	const double *ref_xyz, *input_xyz, *charge, *rot_move, *rot_unit;
-	const double *reqm, *vA, *vB, *vC, *vD, *solpar, *volume;
 	const unsigned long long* rot_mask;
-	const float *r6, *r10, *r12, *repsr, *desolv, *qasp_absq;
-	const int *type, *map, *vwidx;
-	const unsigned char *ignore, *is_hb;
-	const unsigned int* pairs;
+	const float4* rtab;                    // (1/r^6, 1/r^10, 1/r^12, -) of the distance tables
+	const float2* etab;                    // (elec factor, desolvation gaussian)
+	const int *type, *map;
+	const unsigned char* ignore;
+	const struct PostPair* pairs;
 	double movvec[3];                      // get_movvec_to_origo of the reference orientation
 	double spacing, origin[3];
 	float smooth, elec_min_distance;
+};
+
+// One intramolecular contributor with its type-pair parameters and charge
+// products resolved on the host in the reference's operations.
+struct __align__(16) PostPair {
+	double v12, vn;                        // vw_A, vw_B, or vw_C, vw_D of an H-bond pair
+	float opt, q1q2, sv;                   // reqm; charge product; s1*w2 + s2*w1 of the desolvation
+	unsigned int ij;                       // i | j << 8 | H-bond << 16 | CG-G0 << 17 | ligand-flexres << 18
 };
 
 struct RunRec {                            // per run, written by the rescoring of its best entity
@@ -63,14 +72,26 @@ struct RunRec {                            // per run, written by the rescoring 
 // separately; each entity's destination is its rank inside its NaN-free
 // segment (ties keep their order).
 // ---------------------------------------------------------------------------
-__device__ int stable_rank(const float* e, int n, int i)
+template <class T>
+__device__ int stable_rank(const T* e, int n, int i)
 {
-	const float x = e[i];
+	const T x = e[i];
 	if (isnan(x)) return i;
 	int s = i;
 	while (s > 0 && !isnan(e[s - 1])) s--;
 	int rank = s;
 	for (int j = s; j < n && !isnan(e[j]); j++) rank += (e[j] < x) || (e[j] == x && j < i);
+	return rank;
+}
+
+// The rank in an array without NaN: one segment, no test per step.
+template <class T>
+__device__ int plain_rank(const T* e, int n, int i)
+{
+	const T x = e[i];
+	int rank = 0;
+#pragma unroll 4
+	for (int j = 0; j < n; j++) rank += (e[j] < x) || (e[j] == x && j < i);
 	return rank;
 }
 
@@ -80,16 +101,21 @@ __global__ void __launch_bounds__(256) arrange_kernel(float* pop, float* energie
 	int* dst = reinterpret_cast<int*>(sh_e + P);
 	const size_t r = blockIdx.x;
 	float* E = energies + r * P;
-	float* G = pop + r * P * 64;
-	float* S = scratch + r * P * 64;
-	for (int i = threadIdx.x; i < P; i += blockDim.x) sh_e[i] = E[i];
+	float4* G = reinterpret_cast<float4*>(pop + r * P * 64);
+	float4* S = reinterpret_cast<float4*>(scratch + r * P * 64);
+	int nans = 0;
+	for (int i = threadIdx.x; i < P; i += blockDim.x) {
+		const float e = E[i];
+		sh_e[i] = e;
+		nans |= isnan(e);
+	}
+	nans = __syncthreads_or(nans);
+	for (int i = threadIdx.x; i < P; i += blockDim.x) dst[i] = nans ? stable_rank(sh_e, P, i) : plain_rank(sh_e, P, i);
 	__syncthreads();
-	for (int i = threadIdx.x; i < P; i += blockDim.x) dst[i] = stable_rank(sh_e, P, i);
-	__syncthreads();
-	for (int k = threadIdx.x; k < P * 64; k += blockDim.x) S[(size_t)dst[k >> 6] * 64 + (k & 63)] = G[k];
+	for (int k = threadIdx.x; k < P * 16; k += blockDim.x) S[dst[k >> 4] * 16 + (k & 15)] = G[k];
 	for (int i = threadIdx.x; i < P; i += blockDim.x) E[dst[i]] = sh_e[i];
 	__syncthreads();
-	for (int k = threadIdx.x; k < P * 64; k += blockDim.x) G[k] = S[k];
+	for (int k = threadIdx.x; k < P * 16; k += blockDim.x) G[k] = S[k];
 }
 
 // ---------------------------------------------------------------------------
@@ -126,29 +152,30 @@ __device__ __forceinline__ double dist2(const double* a, const double* b)
 
 // calc_rmsd (host/src/processligand.cpp:1441-1489) of pose xyz against ref:
 // with symmetry, each atom's squared distance to the nearest reference atom
-// of its type (100000 when there is none).  Per-atom terms in parallel, the
-// sum in atom order on lane 0, the result broadcast to the warp.
-__device__ double warp_rmsd(const double* xyz, const double* ref, const int* type, int n, int symmetry, int lane)
+// of its type (100000 when there is none).  Per-atom terms in parallel into
+// the warp's scratch `terms` (n doubles), the sum in atom order on lane 0,
+// the result broadcast to the warp.
+__device__ double warp_rmsd(const double* xyz, const double* ref, const int* type, int n, int symmetry, int lane,
+                            double* terms)
 {
-	double sum = 0.0;
-	for (int base = 0; base < n; base += 32) {
-		const int a = base + lane;
-		double m = 0.0;
-		if (a < n) {
-			if (symmetry) {
-				m = 100000;
-				for (int b = 0; b < n; b++)
-					if (type[a] == type[b]) {
-						const double d2 = dist2(xyz + 3 * a, ref + 3 * b);
-						if (d2 < m) m = d2;
-					}
-			} else m = dist2(xyz + 3 * a, ref + 3 * a);
-		}
-		for (int k = 0; k < 32; k++) {
-			const double mk = __shfl_sync(0xffffffffu, m, k);
-			if (lane == 0 && base + k < n) sum += mk;
-		}
+	for (int a = lane; a < n; a += 32) {
+		double m;
+		if (symmetry) {
+			const int ta = type[a];
+			m = 100000;
+			for (int b = 0; b < n; b++)
+				if (ta == type[b]) {
+					const double d2 = dist2(xyz + 3 * a, ref + 3 * b);
+					if (d2 < m) m = d2;
+				}
+		} else m = dist2(xyz + 3 * a, ref + 3 * a);
+		terms[a] = m;
 	}
+	__syncwarp();
+	double sum = 0.0;
+	if (lane == 0)
+		for (int a = 0; a < n; a++) sum += terms[a];
+	__syncwarp();
 	return __shfl_sync(0xffffffffu, sqrt(sum / (unsigned)n), 0);
 }
 
@@ -157,18 +184,50 @@ __device__ double warp_rmsd(const double* xyz, const double* ref, const int* typ
 // (host/src/processresult.cpp:421-475): change_conform_f, calc_interE_f in
 // grid units, scale_ligand to Angstrom, calc_intraE_f, move_ligand to the
 // grid's origin, calc_rmsd.  Per-atom and per-pair terms are computed by the
-// lanes; the energies are summed on lane 0 in the reference's atom and pair
-// order, so the float sums round as the host's do.
+// lanes, and each energy is summed by one lane in the reference's atom and
+// pair order, so the float sums round as the host's do.  A term that the
+// reference does not add to a sum is staged as +0, which leaves the sum as it
+// is.  What bounds it: those sums are the only serial part, so the lanes stage
+// 32 entries of each sum in shared memory (rows of 36 floats: four rows read
+// by four lanes fall in different banks) and one lane per sum reads them four
+// at a time, about 45 instructions for 32 pairs.  (Handing every term to lane
+// 0 by shuffles took five shuffles and the branches of the accumulators for
+// each pair, 600 instructions for 32 pairs.)  15,000 entities of the 45-atom,
+// 777-pair ligand: 0.75 ms before; the whole call 5.48 -> 0.71 ms on B200, of
+// which the clustering was 4.2 ms.
 // ---------------------------------------------------------------------------
+constexpr int kRow = 36;                   // floats of a staged row
+constexpr int kRows = 5;
+
+// Adds row `lane`'s 32 staged terms, in order, to the lane's sum (lanes 0..nsum-1).
+__device__ __forceinline__ void add_row(const float* st, int lane, int nsum, float& sum)
+{
+	if (lane >= nsum) return;
+	const float4* row = reinterpret_cast<const float4*>(st + lane * kRow);
+	for (int k = 0; k < 8; k++) {
+		const float4 v = row[k];
+		sum += v.x; sum += v.y; sum += v.z; sum += v.w;
+	}
+}
+
+__host__ __device__ inline size_t rescore_warp_bytes(int N, int NR)
+{
+	// coordinates, sines and cosines, per-atom RMSD terms; staged rows
+	return ((size_t)(4 * N + 2 * NR + 8) * sizeof(double) + 15) / 16 * 16 + (size_t)kRows * kRow * sizeof(float);
+}
+
 __global__ void __launch_bounds__(kWarps * 32)
 rescore_kernel(PostDev D, const float* pop, const float* energies, int ntask, RunRec* runs, double* best_xyz,
                float* peratom, float* entities)
 {
-	extern __shared__ double sh_w[];
+	extern __shared__ __align__(16) unsigned char sh_w[];
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	const int N = D.N, NL = D.NL, NR = D.NR;
-	double* xyz = sh_w + (size_t)warp * (3 * N + 2 * NR + 8);
+	const size_t wb = rescore_warp_bytes(N, NR);
+	double* xyz = reinterpret_cast<double*>(sh_w + (size_t)warp * wb);
 	double* trig = xyz + 3 * N;                // cos, sin of each torsion's half angle; genrot axis, cos, sin
+	double* terms = trig + 2 * NR + 8;         // N
+	float* st = reinterpret_cast<float*>(sh_w + (size_t)(warp + 1) * wb) - kRows * kRow;
 	const size_t g3_4 = ((size_t)D.gx * D.gy * D.gz) << 2;
 	for (int task = blockIdx.x * kWarps + warp; task < ntask; task += gridDim.x * kWarps) {
 		const int run = D.rescore_all ? task / D.P : task;
@@ -210,7 +269,7 @@ rescore_kernel(PostDev D, const float* pop, const float* energies, int ntask, Ru
 
 		// calc_interE_f (host/src/processligand.cpp:1796-2055)
 		const bool best = ent == 0;
-		float interE = 0.0f, intraflexE = 0.0f, elecE = 0.0f;
+		float isum = 0.0f;                     // lane 0: interE, lane 1: intraflexE, lane 2: elecE
 		for (int base = 0; base < N; base += 32) {
 			const int a = base + lane;
 			int kind = 0;                      // 0: not counted, 1: outside the grid, 2: interpolated
@@ -276,16 +335,17 @@ rescore_kernel(PostDev D, const float* pop, const float* energies, int ntask, Ru
 				pa[0] = kind == 2 ? vd : (kind == 1 ? 100000.0f : 0.0f);
 				pa[1] = kind == 2 ? e : (kind == 1 ? 100000.0f : 0.0f);
 			}
-			for (int k = 0; k < 32; k++) {
-				const float vk = __shfl_sync(0xffffffffu, val, k), ek = __shfl_sync(0xffffffffu, e, k);
-				const int kk = __shfl_sync(0xffffffffu, kind, k);
-				if (lane == 0 && kk) {
-					if (base + k < NL) interE += vk;
-					else intraflexE += vk;
-					if (kk == 2 && base + k < NL) elecE += ek;
-				}
-			}
+			const bool lig = a < NL;
+			st[lane] = kind && lig ? val : 0.0f;
+			st[kRow + lane] = kind && !lig ? val : 0.0f;
+			st[2 * kRow + lane] = kind == 2 && lig ? e : 0.0f;
+			__syncwarp();
+			add_row(st, lane, 3, isum);
+			__syncwarp();
 		}
+		const float interE = __shfl_sync(0xffffffffu, isum, 0);
+		const float intraflexE = __shfl_sync(0xffffffffu, isum, 1);
+		const float elecE = __shfl_sync(0xffffffffu, isum, 2);
 
 		// scale_ligand to Angstrom (the grid's spacing)
 		for (int a = lane; a < N; a += 32)
@@ -294,41 +354,31 @@ rescore_kernel(PostDev D, const float* pop, const float* energies, int ntask, Ru
 
 		// calc_intraE_f (host/src/processligand.cpp:2058-2331), without
 		// modified pairs (the front end has none) and without contact analysis
-		float vW = 0.0f, el = 0.0f, desolv = 0.0f, interflexE = 0.0f;
+		float psum = 0.0f;                     // lane 0: vW, lane 1: elec, lane 2: desolv, lane 3: interflexE
 		const float delta = 0.5f * D.smooth;
 		for (int base = 0; base < D.Q; base += 32) {
 			const int pi = base + lane;
-			int fl = 0;                         // 1: CG-G0 term, 2: vdW/H-bond term, 4: elec+desolv, 8: ligand-flexres pair
+			bool flex = false;
 			float t_cg = 0.0f, t_vdw = 0.0f, t_a = 0.0f, t_b = 0.0f;
 			if (pi < D.Q) {
-				const int i = (int)D.pairs[2 * pi], j = (int)D.pairs[2 * pi + 1];
-				if (((i >= NL) + (j >= NL)) & 1) fl |= 8;
+				const PostPair pp = D.pairs[pi];
+				const int i = (int)(pp.ij & 0xFFu), j = (int)((pp.ij >> 8) & 0xFFu);
+				flex = (pp.ij >> 18) & 1u;
 				float dist = (float)sqrt(dist2(xyz + 3 * i, xyz + 3 * j));
 				int did = (int)floorf((100.0f * dist) + 0.5f) - 1;
 				if (did < 0) did = 0;
-				const int t1 = D.type[i], t2 = D.type[j], tp = t1 * D.NT + t2;
-				const int v1 = D.vwidx[t1], v2 = D.vwidx[t2];
-				if ((v1 == kCG && v2 == kG0) || (v1 == kG0 && v2 == kCG)) {
-					fl |= 1;
-					t_cg = kGbond * dist;
-				}
+				if ((pp.ij >> 17) & 1u) t_cg = kGbond * dist;
 				if (dist < kDcutoff) {
-					const float opt = (float)D.reqm[tp];
+					const float opt = pp.opt;
 					float sd;
 					if (dist <= (opt - delta)) sd = dist + delta;
 					else if (dist < (opt + delta)) sd = opt;
 					else sd = dist - delta;
 					int sid = (int)floorf((100.0f * sd) + 0.5f) - 1;
 					if (sid < 0) sid = 0;
-					float vdw1, vdw2;
-					if (D.is_hb[tp]) {
-						vdw1 = (float)(D.vC[tp] * D.r12[sid]);
-						vdw2 = (float)(D.vD[tp] * D.r10[sid]);
-					} else {
-						vdw1 = (float)(D.vA[tp] * D.r12[sid]);
-						vdw2 = (float)(D.vB[tp] * D.r6[sid]);
-					}
-					fl |= 2;
+					const float4 rt = D.rtab[sid];
+					const float vdw1 = (float)(pp.v12 * rt.z);
+					const float vdw2 = (float)(pp.vn * ((pp.ij >> 16) & 1u ? rt.y : rt.x));
 					t_vdw = vdw1 - vdw2;
 				}
 				if (dist < 20.48) {
@@ -339,32 +389,28 @@ rescore_kernel(PostDev D, const float* pop, const float* energies, int ntask, Ru
 						// the reference reads outside its table here when elec_min_distance < 0.005
 						eid = eid < 0 ? 0 : (eid >= kTab ? kTab - 1 : eid);
 					}
-					const float s1 = (float)(D.solpar[t1] + D.qasp_absq[i]);
-					const float s2 = (float)(D.solpar[t2] + D.qasp_absq[j]);
-					const float w1 = (float)D.volume[t1], w2 = (float)D.volume[t2];
-					const float q1q2 = (float)((double)(float)D.charge[i] * D.charge[j]);
-					t_a = q1q2 * D.repsr[eid];
-					t_b = (s1 * w2 + s2 * w1) * D.desolv[eid];
-					fl |= 4;
+					const float2 et = D.etab[eid];
+					t_a = pp.q1q2 * et.x;
+					t_b = pp.sv * et.y;
 				}
 			}
-			for (int k = 0; k < 32; k++) {
-				const int fk = __shfl_sync(0xffffffffu, fl, k);
-				const float ck = __shfl_sync(0xffffffffu, t_cg, k), vk = __shfl_sync(0xffffffffu, t_vdw, k);
-				const float ak = __shfl_sync(0xffffffffu, t_a, k), bk = __shfl_sync(0xffffffffu, t_b, k);
-				if (lane == 0 && fk) {
-					const bool flex = fk & 8;
-					// the CG-G0 term goes the other way round from the others
-					// (host/src/processligand.cpp:2142-2145)
-					if (fk & 1) { if (flex) vW += ck; else interflexE += ck; }
-					if (fk & 2) { if (flex) interflexE += vk; else vW += vk; }
-					if (fk & 4) {
-						if (flex) interflexE += ak + bk;
-						else { el += ak; desolv += bk; }
-					}
-				}
+			// a ligand-flexres pair's terms go to interflexE, all but its CG-G0
+			// term, which goes the other way round (host/src/processligand.cpp:2142-2145)
+			st[lane] = flex ? t_cg : t_vdw;
+			st[kRow + lane] = flex ? 0.0f : t_a;
+			st[2 * kRow + lane] = flex ? 0.0f : t_b;
+			if (D.flex_or_cg) {
+				st[3 * kRow + lane] = flex ? t_vdw : t_cg;
+				st[4 * kRow + lane] = flex ? t_a + t_b : 0.0f;
 			}
+			__syncwarp();
+			add_row(st, lane, 3, psum);
+			if (D.flex_or_cg && lane == 3)
+				for (int k = 0; k < 32; k++) { psum += st[3 * kRow + k]; psum += st[4 * kRow + k]; }
+			__syncwarp();
 		}
+		const float vW = __shfl_sync(0xffffffffu, psum, 0), el = __shfl_sync(0xffffffffu, psum, 1);
+		const float desolv = __shfl_sync(0xffffffffu, psum, 2), interflexE = __shfl_sync(0xffffffffu, psum, 3);
 		const float intraE = vW + el + desolv;
 
 		// move_ligand by the grid's origin (ligand and flexible residues)
@@ -373,7 +419,7 @@ rescore_kernel(PostDev D, const float* pop, const float* energies, int ntask, Ru
 		__syncwarp();
 		double rmsd = 0.0;
 		if (best || D.rescore_all)
-			rmsd = warp_rmsd(xyz, D.input_xyz, D.type, D.rmsd_atoms, D.symmetry, lane);
+			rmsd = warp_rmsd(xyz, D.input_xyz, D.type, D.rmsd_atoms, D.symmetry, lane, terms);
 		if (lane == 0) {
 			if (entities) {
 				float* o = entities + ((size_t)run * D.P + ent) * 3;
@@ -400,43 +446,158 @@ rescore_kernel(PostDev D, const float* pop, const float* energies, int ntask, Ru
 // 688-804): runs ordered by energy (inter + interflex, plus intra terms for
 // flexible residues alone) with the same NaN-segment stable ranking; then
 // each run in that order joins the first cluster whose centre (its first
-// member) lies within the RMSD tolerance, or founds a new one.  The RMSDs to
-// all current centres are taken in parallel (one warp per centre); the scan
-// over runs stays in order.  Cluster statistics: one thread per cluster.
+// member) lies within the RMSD tolerance, or founds a new one.
+//
+// The scan over runs is serial, so what it needs per run is made small: the
+// RMSDs of all pairs (later run, earlier run) are taken beforehand over the
+// whole GPU (pair_rmsd_kernel), as one bit each for "within the tolerance",
+// and one warp scans the rows.  Centres are founded in run order, so the first
+// cluster within the tolerance is the lowest set bit of row & centres.  That
+// needs R^2/2 RMSDs instead of one per run and centre, so it serves up to
+// kPairRuns runs (4 MB of RMSDs); above it cluster_kernel takes the RMSDs to
+// the current centres as it goes, one warp per centre.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024)
-cluster_kernel(PostDev D, int R, RunRec* runs, const double* best_xyz, double* en, int* order, int* centers,
-               double* crmsd, double tol, int calc, int ncp, int free_roaming, double torsional,
-               adgpu_cluster* clusters, int* nclus)
+constexpr int kPairRuns = 1024;
+
+__device__ double run_energy(const RunRec& r, int free_roaming)
 {
-	__shared__ int s_found, s_K;
-	__shared__ double s_rmsd;
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+	double e = (double)(r.inter + r.interflex);
+	if (!free_roaming) e += (double)(r.intra + r.intraflex);
+	return e;
+}
+
+// Energy order of the runs.  Launch with 1024 threads.
+__global__ void __launch_bounds__(1024) order_kernel(int R, RunRec* runs, double* en, int* order, int free_roaming)
+{
+	__shared__ double s_en[kPairRuns];
+	const int tid = threadIdx.x;
+	double* const E = R <= kPairRuns ? s_en : en;
+	int nans = 0;
 	for (int r = tid; r < R; r += blockDim.x) {
-		double e = (double)(runs[r].inter + runs[r].interflex);
-		if (!free_roaming) e += (double)(runs[r].intra + runs[r].intraflex);
-		en[r] = e;
+		E[r] = run_energy(runs[r], free_roaming);
+		nans |= isnan(E[r]);
 	}
-	__syncthreads();
+	nans = __syncthreads_or(nans);
 	for (int r = tid; r < R; r += blockDim.x) {
-		double x = en[r];
-		int rank;
-		if (isnan(x)) rank = r;
-		else {
-			int s = r;
-			while (s > 0 && !isnan(en[s - 1])) s--;
-			rank = s;
-			for (int j = s; j < R && !isnan(en[j]); j++) rank += (en[j] < x) || (en[j] == x && j < r);
-		}
+		const int rank = nans ? stable_rank(E, R, r) : plain_rank(E, R, r);
 		order[rank] = r;
 		runs[r].rank = rank;
 	}
-	__syncthreads();
-	if (!calc) {
-		if (tid == 0) *nclus = 0;
-		return;
+}
+
+// RMSD of the w-th run in energy order from the u-th, u < w, for every pair
+// p = w (w - 1) / 2 + u: one warp each.
+__global__ void __launch_bounds__(kWarps * 32)
+pair_rmsd_kernel(PostDev D, int R, const double* best_xyz, const int* order, double tol, float* mat, unsigned int* bits)
+{
+	extern __shared__ __align__(16) unsigned char sh_w[];
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = D.rmsd_atoms, N = D.N, W = (R + 31) / 32;
+	double* terms = reinterpret_cast<double*>(sh_w) + (size_t)warp * N;
+	const int npair = R * (R - 1) / 2;
+	for (int p = blockIdx.x * kWarps + warp; p < npair; p += gridDim.x * kWarps) {
+		int w = (int)((1.0 + sqrt(1.0 + 8.0 * (double)p)) * 0.5);
+		while (w * (w - 1) / 2 > p) w--;
+		while (w * (w + 1) / 2 <= p) w++;
+		const int u = p - w * (w - 1) / 2;
+		const double d = warp_rmsd(best_xyz + (size_t)order[w] * N * 3, best_xyz + (size_t)order[u] * N * 3, D.type, n,
+		                           D.symmetry, lane, terms);
+		if (lane == 0) {
+			mat[(size_t)w * R + u] = (float)d;
+			if (d <= tol) atomicOr(bits + (size_t)w * W + (u >> 5), 1u << (u & 31));
+		}
+		__syncwarp();
 	}
+}
+
+// Cluster statistics of cluster c (host/src/processresult.cpp:748-804), its
+// members in energy order; clus_of(u) is the cluster of the u-th run in order.
+template <class F>
+__device__ void cluster_stats(int c, int R, RunRec* runs, const int* order, int ncp, int free_roaming, double torsional,
+                              adgpu_cluster* clusters, F clus_of)
+{
+	int sub = 0;
+	double sum = 0.0, bestE = 0.0;
+	int best_run = 0;
+	for (int u = 0; u < R; u++) {
+		if (clus_of(u) != c + 1) continue;
+		const int j = order[u];
+		sub++;
+		sum += runs[j].inter + runs[j].interflex + torsional;
+		if (!free_roaming) sum += runs[j].intra + runs[j].intraflex;
+		runs[j].subrank = sub;
+		runs[j].output = !((ncp > 0) && (sub > ncp)) && (ncp >= 0);
+		if (sub == 1) {
+			bestE = runs[j].inter + runs[j].interflex + torsional;
+			if (!free_roaming) bestE += runs[j].intra + runs[j].intraflex;
+			best_run = j + 1;
+			runs[j].output = 1;
+		}
+	}
+	clusters[c].size = sub;
+	clusters[c].best_run = best_run;
+	clusters[c].best_energy = bestE;
+	clusters[c].sum_energy = sum;
+}
+
+// The scan over the rows of pair_rmsd_kernel and the cluster statistics, R <=
+// kPairRuns.  Dynamic shared memory: the rows.
+__global__ void __launch_bounds__(256)
+cluster_scan_kernel(int R, RunRec* runs, const int* order, const float* mat, const unsigned int* bits, int ncp,
+                    int free_roaming, double torsional, adgpu_cluster* clusters, int* nclus)
+{
+	extern __shared__ unsigned int s_bits[];
+	__shared__ short s_clus[kPairRuns], s_centre[kPairRuns];
+	__shared__ int s_K;
+	const int tid = threadIdx.x, lane = tid & 31, W = (R + 31) / 32;
+	for (int k = tid; k < R * W; k += blockDim.x) s_bits[k] = bits[k];
+	__syncthreads();
+	if (tid < 32) {
+		unsigned int centres = 0;          // lane l: runs 32 l .. 32 l + 31
+		int K = 0;
+		for (int w = 0; w < R; w++) {
+			const unsigned int m = lane < W ? s_bits[w * W + lane] & centres : 0u;
+			const unsigned int any = __ballot_sync(0xffffffffu, m != 0u);
+			int u = w;
+			if (any) {
+				const int l = __ffs(any) - 1;
+				u = 32 * l + __ffs(__shfl_sync(0xffffffffu, m, l)) - 1;
+			} else {
+				K++;
+				if (lane == (w >> 5)) centres |= 1u << (w & 31);
+			}
+			if (lane == 0) {
+				s_centre[w] = (short)u;
+				s_clus[w] = u == w ? (short)K : s_clus[u];
+			}
+		}
+		if (lane == 0) s_K = K;
+	}
+	__syncthreads();
+	for (int w = tid; w < R; w += blockDim.x) {
+		RunRec& r = runs[order[w]];
+		r.clus = s_clus[w];
+		r.crmsd = s_centre[w] == w ? 0.0f : mat[(size_t)w * R + s_centre[w]];
+	}
+	const int K = s_K;
+	for (int c = tid; c < K; c += blockDim.x)
+		cluster_stats(c, R, runs, order, ncp, free_roaming, torsional, clusters, [&](int u) { return (int)s_clus[u]; });
+	if (tid == 0) *nclus = K;
+}
+
+// More than kPairRuns runs: the RMSDs to all current centres taken in
+// parallel (one warp per centre) for each run in turn.  Dynamic shared memory:
+// N doubles per warp.
+__global__ void __launch_bounds__(1024)
+cluster_kernel(PostDev D, int R, RunRec* runs, const double* best_xyz, const int* order, int* centers,
+               double* crmsd, double tol, int ncp, int free_roaming, double torsional,
+               adgpu_cluster* clusters, int* nclus)
+{
+	extern __shared__ __align__(16) unsigned char sh_w[];
+	__shared__ int s_found, s_K;
+	__shared__ double s_rmsd;
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
 	const int n = D.rmsd_atoms, N = D.N;
+	double* terms = reinterpret_cast<double*>(sh_w) + (size_t)warp * N;
 	if (tid == 0) {
 		const int c0 = order[0];
 		runs[c0].clus = 1;
@@ -448,9 +609,12 @@ cluster_kernel(PostDev D, int R, RunRec* runs, const double* best_xyz, double* e
 	for (int w = 1; w < R; w++) {
 		const int i = order[w];
 		const int K = s_K;
-		for (int c = warp; c < K; c += nwarps)
-			crmsd[c] = warp_rmsd(best_xyz + (size_t)i * N * 3, best_xyz + (size_t)centers[c] * N * 3, D.type, n,
-			                     D.symmetry, lane);
+		for (int c = warp; c < K; c += nwarps) {
+			const double d = warp_rmsd(best_xyz + (size_t)i * N * 3, best_xyz + (size_t)centers[c] * N * 3, D.type, n,
+			                           D.symmetry, lane, terms);
+			if (lane == 0) crmsd[c] = d;
+			__syncwarp();
+		}
 		__syncthreads();
 		if (tid == 0) {
 			int f = -1;
@@ -474,30 +638,8 @@ cluster_kernel(PostDev D, int R, RunRec* runs, const double* best_xyz, double* e
 		__syncthreads();
 	}
 	const int K = s_K;
-	for (int c = tid; c < K; c += blockDim.x) {
-		int sub = 0;
-		double sum = 0.0, bestE = 0.0;
-		int best_run = 0;
-		for (int u = 0; u < R; u++) {
-			const int j = order[u];
-			if (runs[j].clus != c + 1) continue;
-			sub++;
-			sum += runs[j].inter + runs[j].interflex + torsional;
-			if (!free_roaming) sum += runs[j].intra + runs[j].intraflex;
-			runs[j].subrank = sub;
-			runs[j].output = !((ncp > 0) && (sub > ncp)) && (ncp >= 0);
-			if (sub == 1) {
-				bestE = runs[j].inter + runs[j].interflex + torsional;
-				if (!free_roaming) bestE += runs[j].intra + runs[j].intraflex;
-				best_run = j + 1;
-				runs[j].output = 1;
-			}
-		}
-		clusters[c].size = sub;
-		clusters[c].best_run = best_run;
-		clusters[c].best_energy = bestE;
-		clusters[c].sum_energy = sum;
-	}
+	for (int c = tid; c < K; c += blockDim.x)
+		cluster_stats(c, R, runs, order, ncp, free_roaming, torsional, clusters, [&](int u) { return runs[order[u]].clus; });
 	if (tid == 0) *nclus = K;
 }
 
@@ -517,19 +659,29 @@ double ddd_mehler_solmajer(double d)
 	return eps;
 }
 
-void distance_tables(float* r6, float* r10, float* r12, float* repsr, float* desolv, float coeff_elec, float coeff_desolv)
-{
-	float dist = 0;
-	const float sigma = 3.6f;
-	for (int i = 0; i < kTab; i++) {
-		dist += 0.01;
-		r6[i] = 1 / powf(dist, 6);
-		r10[i] = 1 / powf(dist, 10);
-		r12[i] = 1 / powf(dist, 12);
-		repsr[i] = (float)coeff_elec / (dist * ddd_mehler_solmajer(dist));
-		desolv[i] = coeff_desolv * expf(-1 * dist * dist / (2 * sigma * sigma));
+// What the tables hold apart from the two coefficients is the same for every
+// ligand and is made once.
+struct DistanceTables {
+	float4 r[kTab];
+	double eps_r[kTab];                    // dist * dielectric
+	float gauss[kTab];
+	DistanceTables()
+	{
+		float dist = 0;
+		const float sigma = 3.6f;
+		for (int i = 0; i < kTab; i++) {
+			dist += 0.01;
+			r[i] = make_float4(1 / powf(dist, 6), 1 / powf(dist, 10), 1 / powf(dist, 12), 0.0f);
+			eps_r[i] = dist * ddd_mehler_solmajer(dist);
+			gauss[i] = expf(-1 * dist * dist / (2 * sigma * sigma));
+		}
 	}
-}
+	static const DistanceTables& get()
+	{
+		static const DistanceTables t;
+		return t;
+	}
+};
 
 template <class T>
 size_t put(std::vector<unsigned char>& blob, const T* src, size_t n)
@@ -581,31 +733,49 @@ adgpu_status process_result_core(const PostLigand& L, const uint32_t* pairs, con
 	const int N = L.natoms, NR = L.nrot, NT = L.ntypes, P = dp.pop_size, R = (int)num_runs;
 	const int Q = dp.num_of_intraE_contributors;
 
-	// host side: constant tables (IntraTables) and the packed ligand
-	std::vector<float> tab(5 * kTab);
-	distance_tables(tab.data(), tab.data() + kTab, tab.data() + 2 * kTab, tab.data() + 3 * kTab, tab.data() + 4 * kTab,
-	                dp.coeff_elec, dp.coeff_desolv);
+	// host side: constant tables (IntraTables), the pairs and the packed ligand
+	const DistanceTables& T = DistanceTables::get();
+	std::vector<float2> etab(kTab);
+	for (int i = 0; i < kTab; i++) etab[i] = make_float2((float)(dp.coeff_elec / T.eps_r[i]), dp.coeff_desolv * T.gauss[i]);
 	std::vector<float> qabs(N);
 	for (int i = 0; i < N; i++) qabs[i] = dp.qasp * fabs(L.charge[i]);        // calc_q_tables_f
+	std::vector<PostPair> pp(Q);
+	bool flex_or_cg = false;
+	for (int k = 0; k < Q; k++) {
+		const int i = (int)pairs[2 * k], j = (int)pairs[2 * k + 1], t1 = L.type[i], t2 = L.type[j], tp = t1 * NT + t2;
+		const int v1 = L.vw_index[t1], v2 = L.vw_index[t2];
+		const bool hb = L.is_hb[tp] != 0, cg = (v1 == kCG && v2 == kG0) || (v1 == kG0 && v2 == kCG);
+		const bool flex = ((i >= L.true_lig_atoms) + (j >= L.true_lig_atoms)) & 1;
+		const float s1 = (float)(L.solpar[t1] + qabs[i]), s2 = (float)(L.solpar[t2] + qabs[j]);
+		const float w1 = (float)L.volume[t1], w2 = (float)L.volume[t2];
+		pp[k].v12 = hb ? L.vw_C[tp] : L.vw_A[tp];
+		pp[k].vn = hb ? L.vw_D[tp] : L.vw_B[tp];
+		pp[k].opt = (float)L.reqm_AB[tp];
+		pp[k].q1q2 = (float)((double)(float)L.charge[i] * L.charge[j]);
+		pp[k].sv = s1 * w2 + s2 * w1;
+		pp[k].ij = (unsigned)i | (unsigned)j << 8 | (unsigned)hb << 16 | (unsigned)cg << 17 | (unsigned)flex << 18;
+		flex_or_cg |= cg || flex;
+	}
 	std::vector<unsigned char> blob;
 	const size_t o_ref = put(blob, L.ref_xyz.data(), 3 * N), o_in = put(blob, L.input_xyz.data(), 3 * N),
 	             o_q = put(blob, L.charge.data(), N), o_mv = put(blob, L.rot_move.data(), 3 * NR),
-	             o_un = put(blob, L.rot_unit.data(), 3 * NR), o_reqm = put(blob, L.reqm_AB.data(), NT * NT),
-	             o_A = put(blob, L.vw_A.data(), NT * NT), o_B = put(blob, L.vw_B.data(), NT * NT),
-	             o_C = put(blob, L.vw_C.data(), NT * NT), o_D = put(blob, L.vw_D.data(), NT * NT),
-	             o_sp = put(blob, L.solpar.data(), NT), o_vol = put(blob, L.volume.data(), NT),
-	             o_mask = put(blob, L.rot_mask.data(), N), o_tab = put(blob, tab.data(), tab.size()),
-	             o_qa = put(blob, qabs.data(), N), o_ty = put(blob, L.type.data(), N), o_map = put(blob, L.map.data(), N),
-	             o_vw = put(blob, L.vw_index.data(), NT), o_ig = put(blob, L.ignore_inter.data(), N),
-	             o_hb = put(blob, L.is_hb.data(), NT * NT), o_pr = put(blob, pairs, 2 * (size_t)Q);
+	             o_un = put(blob, L.rot_unit.data(), 3 * NR), o_mask = put(blob, L.rot_mask.data(), N),
+	             o_rt = put(blob, T.r, kTab), o_et = put(blob, etab.data(), kTab), o_ty = put(blob, L.type.data(), N),
+	             o_map = put(blob, L.map.data(), N), o_ig = put(blob, L.ignore_inter.data(), N),
+	             o_pr = put(blob, pp.data(), Q);
 	// device scratch
 	const size_t n_pop = (size_t)R * P * 64;
 	size_t off = (blob.size() + 255) / 256 * 256;
 	auto take = [&](size_t bytes) { size_t o = off; off = (off + bytes + 255) / 256 * 256; return o; };
 	const size_t o_scr = take(n_pop * 4), o_runs = take((size_t)R * sizeof(RunRec)), o_bx = take((size_t)R * N * 3 * 8),
 	             o_pa = take((size_t)R * N * 2 * 4), o_ent = take(params->rescore_entities ? (size_t)R * P * 3 * 4 : 0),
-	             o_en = take((size_t)R * 8), o_ord = take((size_t)R * 4), o_cen = take((size_t)R * 4),
-	             o_cr = take((size_t)R * 8), o_cl = take((size_t)R * sizeof(adgpu_cluster)), o_nc = take(4);
+	             o_en = take((size_t)R * 8), o_ord = take((size_t)R * 4), o_cl = take((size_t)R * sizeof(adgpu_cluster)),
+	             o_nc = take(4);
+	// clustering: the pairs' RMSDs and rows, or the centres and their RMSDs
+	const bool by_pairs = R <= kPairRuns;
+	const int W = (R + 31) / 32;
+	const size_t o_cen = take(by_pairs ? (size_t)R * R * 4 : (size_t)R * 4),
+	             o_cr = take(by_pairs ? (size_t)R * W * 4 : (size_t)R * 8);
 
 	unsigned char* d = nullptr;
 	auto done = [&](cudaError_t err, const char* what) {
@@ -630,15 +800,11 @@ adgpu_status process_result_core(const PostLigand& L, const uint32_t* pairs, con
 	D.grid = grid;
 	D.ref_xyz = (const double*)(d + o_ref); D.input_xyz = (const double*)(d + o_in); D.charge = (const double*)(d + o_q);
 	D.rot_move = (const double*)(d + o_mv); D.rot_unit = (const double*)(d + o_un);
-	D.reqm = (const double*)(d + o_reqm); D.vA = (const double*)(d + o_A); D.vB = (const double*)(d + o_B);
-	D.vC = (const double*)(d + o_C); D.vD = (const double*)(d + o_D);
-	D.solpar = (const double*)(d + o_sp); D.volume = (const double*)(d + o_vol);
+	D.flex_or_cg = flex_or_cg ? 1 : 0;
 	D.rot_mask = (const unsigned long long*)(d + o_mask);
-	const float* T = (const float*)(d + o_tab);
-	D.r6 = T; D.r10 = T + kTab; D.r12 = T + 2 * kTab; D.repsr = T + 3 * kTab; D.desolv = T + 4 * kTab;
-	D.qasp_absq = (const float*)(d + o_qa);
-	D.type = (const int*)(d + o_ty); D.map = (const int*)(d + o_map); D.vwidx = (const int*)(d + o_vw);
-	D.ignore = d + o_ig; D.is_hb = d + o_hb; D.pairs = (const unsigned int*)(d + o_pr);
+	D.rtab = (const float4*)(d + o_rt); D.etab = (const float2*)(d + o_et);
+	D.type = (const int*)(d + o_ty); D.map = (const int*)(d + o_map);
+	D.ignore = d + o_ig; D.pairs = (const PostPair*)(d + o_pr);
 	// get_movvec_to_origo of the reference orientation (host/src/processligand.cpp:1363-1387)
 	if (L.true_lig_atoms > 0) {
 		double t[3] = {0, 0, 0};
@@ -659,16 +825,44 @@ adgpu_status process_result_core(const PostLigand& L, const uint32_t* pairs, con
 
 	arrange_kernel<<<R, 256, (size_t)P * 8, st>>>(populations, energies, (float*)(d + o_scr), P);
 	const int ntask = params->rescore_entities ? R * P : R;
-	const size_t wsm = (size_t)kWarps * (3 * N + 2 * NR + 8) * sizeof(double);
+	const size_t wsm = (size_t)kWarps * rescore_warp_bytes(N, NR);
+	if (wsm > 48 * 1024) {
+		e = cudaFuncSetAttribute(rescore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
+		if (e != cudaSuccess) return done(e, "result smem");
+	}
 	int dev = 0, sms = 148;
 	cudaGetDevice(&dev);
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 	const int blocks = std::min((ntask + kWarps - 1) / kWarps, sms * 8);
 	rescore_kernel<<<blocks, kWarps * 32, wsm, st>>>(D, populations, energies, ntask, d_runs, d_bx, d_pa, d_ent);
-	cluster_kernel<<<1, 1024, 0, st>>>(D, R, d_runs, d_bx, (double*)(d + o_en), (int*)(d + o_ord), (int*)(d + o_cen),
-	                                   (double*)(d + o_cr), (double)params->rmsd_tolerance, params->calc_clustering ? 1 : 0,
-	                                   params->nr_cluster_poses, params->free_roaming_ligand ? 1 : 0,
-	                                   params->coeff_tors * L.true_lig_rotbonds, d_cl, d_nc);
+	const int free_roaming = params->free_roaming_ligand ? 1 : 0;
+	const double tol = (double)params->rmsd_tolerance, torsional = params->coeff_tors * L.true_lig_rotbonds;
+	int* d_ord = (int*)(d + o_ord);
+	order_kernel<<<1, 1024, 0, st>>>(R, d_runs, (double*)(d + o_en), d_ord, free_roaming);
+	if (!params->calc_clustering) {
+		e = cudaMemsetAsync(d_nc, 0, 4, st);
+	} else if (by_pairs) {
+		float* mat = (float*)(d + o_cen);
+		unsigned int* bits = (unsigned int*)(d + o_cr);
+		const int npair = R * (R - 1) / 2;
+		e = cudaMemsetAsync(bits, 0, (size_t)R * W * 4, st);
+		if (npair > 0)
+			pair_rmsd_kernel<<<std::min((npair + kWarps - 1) / kWarps, sms * 16), kWarps * 32, (size_t)kWarps * N * 8, st>>>(
+			    D, R, d_bx, d_ord, tol, mat, bits);
+		const size_t rows = (size_t)R * W * 4;
+		if (e == cudaSuccess && rows > 40 * 1024)
+			e = cudaFuncSetAttribute(cluster_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows);
+		if (e == cudaSuccess)
+			cluster_scan_kernel<<<1, 256, rows, st>>>(R, d_runs, d_ord, mat, bits, params->nr_cluster_poses, free_roaming,
+			                                          torsional, d_cl, d_nc);
+	} else {
+		const size_t csm = (size_t)32 * N * 8;
+		if (csm > 48 * 1024) e = cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
+		if (e == cudaSuccess)
+			cluster_kernel<<<1, 1024, csm, st>>>(D, R, d_runs, d_bx, d_ord, (int*)(d + o_cen), (double*)(d + o_cr), tol,
+			                                     params->nr_cluster_poses, free_roaming, torsional, d_cl, d_nc);
+	}
+	if (e != cudaSuccess) return done(e, "result clustering");
 	e = cudaGetLastError();
 	if (e != cudaSuccess) return done(e, "result kernels");
 	std::vector<RunRec> h_runs(R);
