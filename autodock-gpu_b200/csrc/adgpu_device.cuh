@@ -154,7 +154,7 @@ struct LigDev {
 	const float4* atom_xyzq;     // reference coordinates (grid units) + charge
 	const uint32_t* atom_info;   // bits 0-7 map-record slot, bit 8 ignore_inter, bit 9 general rotation, bits 16-31 chain start
 	const uint8_t* chain_len;    // torsion rotations per atom
-	const uint8_t* chain;        // torsion ids, per atom, in application order
+	const uint8_t* chain;        // torsion ids, per atom, in application order (each chain from a multiple of 4 on)
 	const float4* tors_uv;       // rotatable bond unit vectors
 	const float4* tors_mv;       // rotatable bond moving vectors
 	const int2* tors_ends;       // rotatable bond atom pair
@@ -310,19 +310,24 @@ struct Group {
 			if (!scratch_free) sync();
 			if ((lane & 3) == 0 && mine < K) red[w * 8 + mine] = w1;
 			sync();
+			// (rows of 8 floats, 16-byte aligned; values past K are not used)
+			float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+			const float4* r4 = reinterpret_cast<const float4*>(red);
 #pragma unroll
-			for (int k = 0; k < K; k++) {
-				float s = 0.0f;
-				for (int i = 0; i < TPP / 32; i++) s += red[i * 8 + k];
-				v[k] = s;
+			for (int i = 0; i < TPP / 32; i++) {
+				const float4 lo = r4[2 * i], hi = K > 4 ? r4[2 * i + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+				s[0] += lo.x; s[1] += lo.y; s[2] += lo.z; s[3] += lo.w;
+				s[4] += hi.x; s[5] += hi.y; s[6] += hi.z; s[7] += hi.w;
 			}
+#pragma unroll
+			for (int k = 0; k < K; k++) v[k] = s[k];
 		}
 	}
 };
 
 // ---- per-pose shared-memory scratch -------------------------------------------------
 // Layout (natoms rounded up to a multiple of 4):
-//   tq [ntors] float4; gsc; xyz [3N] float; f3 [3N] int; gg [64] int
+//   tq [2 ntors] float4 (quaternions, then axes); gsc; xyz [3N] float; f3 [3N] int; gg [64] int
 // An atom's coordinates are xyz[3a .. 3a+2] and its fixed-point force is
 // f3[3a .. 3a+2]: one address per atom for the three components, and since 3
 // is odd, atoms whose indices differ mod 32 fall in different banks, as in
@@ -341,7 +346,7 @@ struct PoseSmem {
 __host__ __device__ inline int pose_smem_bytes(int natoms, int ntors)
 {
 	int n4 = (natoms + 3) & ~3;
-	return (6 * n4) * 4 + ntors * 16 + 32 + 64 * 4;
+	return (6 * n4) * 4 + ntors * 32 + 32 + 64 * 4;
 }
 
 __device__ __forceinline__ PoseSmem carve_pose(char* base, int natoms, int ntors)
@@ -350,7 +355,7 @@ __device__ __forceinline__ PoseSmem carve_pose(char* base, int natoms, int ntors
 	int n4 = (natoms + 3) & ~3;
 	float* f = reinterpret_cast<float*>(base);
 	s.tq = reinterpret_cast<float4*>(f);          // 16-byte aligned first
-	f += ntors * 4;
+	f += ntors * 8;
 	s.gsc = reinterpret_cast<float2*>(f);
 	f += 8;
 	s.xyz = f;                                    // still 16-byte aligned
@@ -486,9 +491,31 @@ __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, i
 	constexpr int kBlock = (int)pair2_block(COUPLED);
 	const float4* pr = L.pairs2 + (rank / 32) * kBlock + (rank % 32);
 	const uint32_t* pw = reinterpret_cast<const uint32_t*>(L.pairs2 + (rank / 32) * kBlock + 96) + (rank % 32);
-	for (int d = rank; d < nrec; d += TPP, pr += (TPP / 32) * kBlock, pw += (TPP / 32) * kBlock * 4) {
-		const uint32_t wa = __ldg(pw), wb = COUPLED ? 0u : __ldg(pw + 32);
-		const float4 q0 = __ldg(pr), q1 = __ldg(pr + 32), q2 = __ldg(pr + 64);
+	// Groups of 128 load a step's record during the step before: they score
+	// few poses per SM, so a step's latency counts, and they have the registers.
+	// (With 64 threads it lost 2 to 4 %.)
+	constexpr bool kAhead = TPP == 128;
+	uint32_t wa = 0, wb = 0;
+	float4 q0, q1, q2;
+	q0 = q1 = q2 = make_float4(0.f, 0.f, 0.f, 0.f);
+	auto load = [&](uint32_t& xa, uint32_t& xb, float4& x0, float4& x1, float4& x2) {
+		xa = __ldg(pw);
+		if (!COUPLED) xb = __ldg(pw + 32);
+		x0 = __ldg(pr); x1 = __ldg(pr + 32); x2 = __ldg(pr + 64);
+		pr += (TPP / 32) * kBlock;
+		pw += (TPP / 32) * kBlock * 4;
+	};
+	uint32_t na = 0, nb = 0;
+	float4 n0, n1, n2;
+	n0 = n1 = n2 = make_float4(0.f, 0.f, 0.f, 0.f);
+	if (kAhead && rank < nrec) load(na, nb, n0, n1, n2);
+	for (int d = rank; d < nrec; d += TPP) {
+		if constexpr (kAhead) {
+			wa = na; wb = nb; q0 = n0; q1 = n1; q2 = n2;
+			if (d + TPP < nrec) load(na, nb, n0, n1, n2);
+		} else {
+			load(wa, wb, q0, q1, q2);
+		}
 		const uint32_t a1 = wa & kPairAtomMask, a2 = (wa >> kPairAtomBits) & kPairAtomMask;
 		const uint32_t b1 = COUPLED ? a1 : (wb & kPairAtomMask);
 		const uint32_t b2 = (COUPLED ? wa >> (2 * kPairAtomBits) : wb >> kPairAtomBits) & kPairAtomMask;
@@ -639,7 +666,9 @@ __device__ __forceinline__ float pair_terms_generic(const LigDev& L, const PoseS
 // ---- the scorer -----------------------------------------------------------------------
 // Scores genotype g (shared memory, read-only here).  Returns the energy (same
 // value in every thread of the group).  With GRAD, writes dE/dgene to
-// grad[0..ngenes) (shared memory).  Leaves the pose coordinates in S.
+// grad[0..ngenes) (shared memory), grad[k] for the thread of rank k mod TPP: a
+// barrier before another thread reads it, and before the next call.  Leaves
+// the pose coordinates in S.
 // REF_GRID: L.grid is the reference's own layout (4 replicated floats per
 // point and map, host/src/processgrid.cpp:244-248) instead of cell records;
 // the same 8 corner values are read, from two 16-byte loads per map.
@@ -647,11 +676,51 @@ __device__ __forceinline__ float pair_terms_generic(const LigDev& L, const PoseS
 // map, electrostatic and desolvation energies, intramolecular vdW/H-bond,
 // electrostatic, desolvation and CG-G0 energies, and the number of atoms
 // outside the grid.
+//
+// What bounds it.  With 32 threads per pose the GPU is full and instructions
+// count (3,690 warp instructions an evaluation of the 45-atom ligand, half of
+// them the pair loop's).  Groups of 64 and 128 threads serve dockings of few
+// runs, where the chain of one evaluation counts: 7,700 cycles at 128 threads
+// and 38 atoms, of which 1,530 were the orientation genes on one warp, 1,600
+// the pose and intermolecular terms, 890 the sines and cosines.  So the three
+// orientation genes, whose formulas differ, go to different warps (64 threads:
+// host loop of 20 runs 37.5 -> 36.2 ms), and with 128 threads the atom tables
+// are loaded ahead of the sines and cosines, and with up to 64 atoms the upper
+// two warps take the intermolecular terms while the lower two, which built
+// the pose, start on the pairs (a docking of one run 24.4 -> 21.0 ms; the
+// early loads lost 2 % at 64 threads and 32).  Every float is computed by the same operations in the same
+// order whatever the group does in parallel, and each thread adds up the same
+// terms: results do not depend on it.
 template <int TPP, bool GRAD, bool REF_GRID = false, bool TERMS = false>
 __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float* __restrict__ grad,
                            const PoseSmem& S, const Group<TPP>& G, float* terms = nullptr)
 {
 	const int rank = G.rank;
+	// the upper half takes the lower half's intermolecular terms
+	constexpr bool kCanSplit = TPP == 128 && !TERMS && !REF_GRID;
+	const bool split = kCanSplit && L.natoms <= TPP / 2;
+
+	// 0. this thread's first atom (with split, the upper half's: its partner's)
+	struct AtomIn { float4 r; uint32_t info, chain; int len; };
+	auto load_atom = [&](int a) {
+		AtomIn x;
+		x.r = L.atom_xyzq[a];
+		x.info = L.atom_info[a];
+		x.len = L.chain_len[a];
+		x.chain = 0;                      // four torsion ids a word (single bytes in the no-allocation tables)
+		if constexpr (!REF_GRID) {
+			if (x.len > 0) x.chain = __ldg(reinterpret_cast<const uint32_t*>(L.chain + (x.info >> 16)));
+		}
+		return x;
+	};
+	constexpr bool kEarly = TPP == 128;
+	const int a0 = split ? rank & (TPP / 2 - 1) : rank;
+	AtomIn in;
+	in.r = make_float4(0.f, 0.f, 0.f, 0.f);
+	in.info = in.chain = 0;
+	in.len = 0;
+	if (kEarly && a0 < L.natoms) in = load_atom(a0);
+
 	// 1. torsion quaternions (cuda/calcMergeEneGra.cu:160-175, computed once per
 	//    torsion) and the sines/cosines of the general rotation, one sincos
 	//    per thread: lanes past the torsions take theta, phi and half the angle
@@ -659,103 +728,109 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 	const int nsc = L.ntors + (has_lig ? 3 : 0);
 	for (int k = rank; k < nsc; k += TPP) {
 		const int j = k - L.ntors;
+		float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+		if (j < 0) u = L.tors_uv[k];
 		const float ang = j < 0 ? g[6 + k] * kDegToRad * 0.5f
 		                        : (j == 0 ? g[4] * kDegToRad : (j == 1 ? g[3] * kDegToRad : g[5] * kDegToRad * 0.5f));
 		float s, c;
 		sincosf(ang, &s, &c);
 		if (j < 0) {
-			float4 u = L.tors_uv[k];
 			S.tq[k] = make_float4(s * u.x, s * u.y, s * u.z, c);
 		} else {
 			S.gsc[j] = make_float2(s, c);
 		}
 	}
-	if (GRAD)
+	if (GRAD && !split)
 		for (int k = rank; k < L.ngenes; k += TPP) S.gg[k] = 0;
 	G.sync();
 	const GenRot gr = genrot_from(g, has_lig, S.gsc);
 
-	// 2. pose: each atom applies its own torsion chain, then the general rotation
-	//    (the per-atom order the reference's rotation list encodes, cuda/calcMergeEneGra.cu:131-190);
-	//    the same thread then takes the atom's intermolecular terms (3.)
 	float e_acc = 0.0f;
 	float tt[TERMS ? 8 : 1] = {0.f};   // TERMS partial sums
+	// 3. intermolecular: trilinear interpolation of the type, e and d maps
+	//    (cuda/calcMergeEneGra.cu:195-413) for an atom at p of charge q; its
+	//    terms go to e_acc, its fixed-point force to (fx, fy, fz)
+	auto inter = [&](float3 p, float q, uint32_t info, int& fx, int& fy, int& fz) {
+		fx = fy = fz = 0;
+		if (info & 0x100u) return;
+		float x = p.x, y = p.y, z = p.z;
+		if (x < 0.f || y < 0.f || z < 0.f || x >= (float)(L.gx - 1) || y >= (float)(L.gy - 1) || z >= (float)(L.gz - 1)) {
+			e_acc += kOutOfGridPenalty;
+			fx = fy = fz = kOutOfGridForce;
+			if constexpr (TERMS) tt[7] += 1.0f;
+			return;
+		}
+		float xl = floorf(x), yl = floorf(y), zl = floorf(z);
+		float dx = x - xl, omdx = 1.0f - dx, dy = y - yl, omdy = 1.0f - dy, dz = z - zl, omdz = 1.0f - dz;
+		float w0 = omdx * omdy * omdz, w1 = omdx * dy * omdz, w2 = omdx * omdy * dz, w3 = omdx * dy * dz;
+		float w4 = dx * omdy * omdz, w5 = dx * dy * omdz, w6 = dx * omdy * dz, w7 = dx * dy * dz;
+		int slot = info & 0xFFu;
+		float4 t0, t1, e0, e1, d0, d1;
+		if constexpr (REF_GRID) {
+			const size_t g3 = (size_t)L.gx * L.gy * L.gz;
+			const size_t p = (size_t)xl + (size_t)yl * L.gx + (size_t)zl * L.gx * L.gy;
+			const size_t M = (size_t)(L.rec_floats / 8 - 2);
+			const float4* tp = reinterpret_cast<const float4*>(L.grid + ((((size_t)slot - 2) * g3 + p) << 2));
+			const float4* ep = reinterpret_cast<const float4*>(L.grid + ((M * g3 + p) << 2));
+			const float4* dp = reinterpret_cast<const float4*>(L.grid + (((M + 1) * g3 + p) << 2));
+			t0 = __ldg(tp); t1 = __ldg(tp + 1); e0 = __ldg(ep); e1 = __ldg(ep + 1); d0 = __ldg(dp); d1 = __ldg(dp + 1);
+		} else {
+			int cell = (int)xl + (int)yl * L.cells_x + (int)zl * L.cells_xy;
+			const float4* rec = reinterpret_cast<const float4*>(L.grid + (size_t)cell * L.rec_floats);
+			t0 = __ldg(rec + 2 * slot); t1 = __ldg(rec + 2 * slot + 1);
+			e0 = __ldg(rec + 0); e1 = __ldg(rec + 1);
+			d0 = __ldg(rec + 2); d1 = __ldg(rec + 3);
+		}
+		float vt = t0.x * w0 + t0.y * w1 + t0.z * w2 + t0.w * w3 + t1.x * w4 + t1.y * w5 + t1.z * w6 + t1.w * w7;
+		float ve = e0.x * w0 + e0.y * w1 + e0.z * w2 + e0.w * w3 + e1.x * w4 + e1.y * w5 + e1.z * w6 + e1.w * w7;
+		float vd = d0.x * w0 + d0.y * w1 + d0.z * w2 + d0.w * w3 + d1.x * w4 + d1.y * w5 + d1.z * w6 + d1.w * w7;
+		e_acc += vt;
+		e_acc += q * ve;
+		e_acc += fabsf(q) * vd;
+		if constexpr (TERMS) { tt[0] += vt; tt[1] += q * ve; tt[2] += fabsf(q) * vd; }
+		if (GRAD) {
+			// corners: .x .y .z .w of rec0 = 000 010 001 011 ; of rec1 = 100 110 101 111
+#define ADGPU_GX(c0, c1) (omdz * (omdy * (c1.x - c0.x) + dy * (c1.y - c0.y)) + dz * (omdy * (c1.z - c0.z) + dy * (c1.w - c0.w)))
+#define ADGPU_GY(c0, c1) (omdz * (omdx * (c0.y - c0.x) + dx * (c1.y - c1.x)) + dz * (omdx * (c0.w - c0.z) + dx * (c1.w - c1.z)))
+#define ADGPU_GZ(c0, c1) (omdy * (omdx * (c0.z - c0.x) + dx * (c1.z - c1.x)) + dy * (omdx * (c0.w - c0.y) + dx * (c1.w - c1.y)))
+			float inv = L.inv_spacing;
+			float gxx = ADGPU_GX(t0, t1) * inv, gyy = ADGPU_GY(t0, t1) * inv, gzz = ADGPU_GZ(t0, t1) * inv;
+			float q1 = q * inv;
+			gxx += q1 * ADGPU_GX(e0, e1); gyy += q1 * ADGPU_GY(e0, e1); gzz += q1 * ADGPU_GZ(e0, e1);
+			q1 = fabsf(q1);
+			gxx += q1 * ADGPU_GX(d0, d1); gyy += q1 * ADGPU_GY(d0, d1); gzz += q1 * ADGPU_GZ(d0, d1);
+#undef ADGPU_GX
+#undef ADGPU_GY
+#undef ADGPU_GZ
+			fx = quant(gxx); fy = quant(gyy); fz = quant(gzz);
+		}
+	};
+
+	// 2. pose: each atom applies its own torsion chain, then the general rotation
+	//    (the per-atom order the reference's rotation list encodes, cuda/calcMergeEneGra.cu:131-190);
+	//    without split the same thread then takes the atom's intermolecular terms
 	for (int a = rank; a < L.natoms; a += TPP) {
-		float4 r4 = L.atom_xyzq[a];
-		float3 p = make_float3(r4.x, r4.y, r4.z);
-		uint32_t info = L.atom_info[a];
-		int cs = info >> 16, cl = L.chain_len[a];
-		for (int i = 0; i < cl; i++) {
-			int k = L.chain[cs + i];
+		if (!kEarly || a != rank) in = load_atom(a);
+		float3 p = make_float3(in.r.x, in.r.y, in.r.z);
+		const int cs = in.info >> 16;
+		uint32_t next = in.chain;
+		for (int i = 0; i < in.len; i++) {
+			if constexpr (REF_GRID) next = L.chain[cs + i];
+			else if (i > 0) next = (i & 3) ? next >> 8 : __ldg(reinterpret_cast<const uint32_t*>(L.chain + cs + i));
+			const int k = (int)(next & 0xFFu);
 			float4 m4 = L.tors_mv[k];
 			float3 m = make_float3(m4.x, m4.y, m4.z);
 			p.x -= m.x; p.y -= m.y; p.z -= m.z;
 			p = qrot(p, S.tq[k]);
 			p.x += m.x; p.y += m.y; p.z += m.z;
 		}
-		if ((info & 0x200u) && a < L.nlig) {
+		if ((in.info & 0x200u) && a < L.nlig) {
 			p = qrot(p, gr.q);
 			p.x += gr.mv.x; p.y += gr.mv.y; p.z += gr.mv.z;
 		}
 		S.xyz[3 * a] = p.x; S.xyz[3 * a + 1] = p.y; S.xyz[3 * a + 2] = p.z;
-
-		// 3. intermolecular: trilinear interpolation of the type, e and d maps
-		//    (cuda/calcMergeEneGra.cu:195-413)
 		int fx = 0, fy = 0, fz = 0;
-		if (!(info & 0x100u)) {
-			float x = p.x, y = p.y, z = p.z;
-			float q = r4.w;
-			if (x < 0.f || y < 0.f || z < 0.f || x >= (float)(L.gx - 1) || y >= (float)(L.gy - 1) || z >= (float)(L.gz - 1)) {
-				e_acc += kOutOfGridPenalty;
-				fx = fy = fz = kOutOfGridForce;
-				if constexpr (TERMS) tt[7] += 1.0f;
-			} else {
-				float xl = floorf(x), yl = floorf(y), zl = floorf(z);
-				float dx = x - xl, omdx = 1.0f - dx, dy = y - yl, omdy = 1.0f - dy, dz = z - zl, omdz = 1.0f - dz;
-				float w0 = omdx * omdy * omdz, w1 = omdx * dy * omdz, w2 = omdx * omdy * dz, w3 = omdx * dy * dz;
-				float w4 = dx * omdy * omdz, w5 = dx * dy * omdz, w6 = dx * omdy * dz, w7 = dx * dy * dz;
-				int slot = info & 0xFFu;
-				float4 t0, t1, e0, e1, d0, d1;
-				if constexpr (REF_GRID) {
-					const size_t g3 = (size_t)L.gx * L.gy * L.gz;
-					const size_t p = (size_t)xl + (size_t)yl * L.gx + (size_t)zl * L.gx * L.gy;
-					const size_t M = (size_t)(L.rec_floats / 8 - 2);
-					const float4* tp = reinterpret_cast<const float4*>(L.grid + ((((size_t)slot - 2) * g3 + p) << 2));
-					const float4* ep = reinterpret_cast<const float4*>(L.grid + ((M * g3 + p) << 2));
-					const float4* dp = reinterpret_cast<const float4*>(L.grid + (((M + 1) * g3 + p) << 2));
-					t0 = __ldg(tp); t1 = __ldg(tp + 1); e0 = __ldg(ep); e1 = __ldg(ep + 1); d0 = __ldg(dp); d1 = __ldg(dp + 1);
-				} else {
-					int cell = (int)xl + (int)yl * L.cells_x + (int)zl * L.cells_xy;
-					const float4* rec = reinterpret_cast<const float4*>(L.grid + (size_t)cell * L.rec_floats);
-					t0 = __ldg(rec + 2 * slot); t1 = __ldg(rec + 2 * slot + 1);
-					e0 = __ldg(rec + 0); e1 = __ldg(rec + 1);
-					d0 = __ldg(rec + 2); d1 = __ldg(rec + 3);
-				}
-				float vt = t0.x * w0 + t0.y * w1 + t0.z * w2 + t0.w * w3 + t1.x * w4 + t1.y * w5 + t1.z * w6 + t1.w * w7;
-				float ve = e0.x * w0 + e0.y * w1 + e0.z * w2 + e0.w * w3 + e1.x * w4 + e1.y * w5 + e1.z * w6 + e1.w * w7;
-				float vd = d0.x * w0 + d0.y * w1 + d0.z * w2 + d0.w * w3 + d1.x * w4 + d1.y * w5 + d1.z * w6 + d1.w * w7;
-				e_acc += vt;
-				e_acc += q * ve;
-				e_acc += fabsf(q) * vd;
-				if constexpr (TERMS) { tt[0] += vt; tt[1] += q * ve; tt[2] += fabsf(q) * vd; }
-				if (GRAD) {
-					// corners: .x .y .z .w of rec0 = 000 010 001 011 ; of rec1 = 100 110 101 111
-#define ADGPU_GX(c0, c1) (omdz * (omdy * (c1.x - c0.x) + dy * (c1.y - c0.y)) + dz * (omdy * (c1.z - c0.z) + dy * (c1.w - c0.w)))
-#define ADGPU_GY(c0, c1) (omdz * (omdx * (c0.y - c0.x) + dx * (c1.y - c1.x)) + dz * (omdx * (c0.w - c0.z) + dx * (c1.w - c1.z)))
-#define ADGPU_GZ(c0, c1) (omdy * (omdx * (c0.z - c0.x) + dx * (c1.z - c1.x)) + dy * (omdx * (c0.w - c0.y) + dx * (c1.w - c1.y)))
-					float inv = L.inv_spacing;
-					float gxx = ADGPU_GX(t0, t1) * inv, gyy = ADGPU_GY(t0, t1) * inv, gzz = ADGPU_GZ(t0, t1) * inv;
-					float q1 = q * inv;
-					gxx += q1 * ADGPU_GX(e0, e1); gyy += q1 * ADGPU_GY(e0, e1); gzz += q1 * ADGPU_GZ(e0, e1);
-					q1 = fabsf(q1);
-					gxx += q1 * ADGPU_GX(d0, d1); gyy += q1 * ADGPU_GY(d0, d1); gzz += q1 * ADGPU_GZ(d0, d1);
-#undef ADGPU_GX
-#undef ADGPU_GY
-#undef ADGPU_GZ
-					fx = quant(gxx); fy = quant(gyy); fz = quant(gzz);
-				}
-			}
-		}
+		if (!split) inter(p, in.r.w, in.info, fx, fy, fz);
 		if (GRAD) {
 			// the start value that cancels couple_force's rounding offsets
 			const unsigned fb = L.f3_bias ? (unsigned)__ldg(L.f3_bias + a) : 0u;
@@ -764,52 +839,97 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 		}
 	}
 	G.sync();
+	if constexpr (kCanSplit) {
+		if (split && rank >= TPP / 2 && a0 < L.natoms) {
+			int fx, fy, fz;
+			inter(ld3(S.xyz + 3 * a0), in.r.w, in.info, fx, fy, fz);
+			reinterpret_cast<float*>(S.gg)[a0] = e_acc;      // its partner's first term
+			e_acc = 0.0f;
+			if (GRAD) {
+				int* fa = S.f3 + 3 * a0;
+				atomicAdd(fa, fx); atomicAdd(fa + 1, fy); atomicAdd(fa + 2, fz);
+			}
+		}
+	}
+	if constexpr (GRAD) {
+		// the torsions' axes for step 6, once per torsion, in place of their
+		// quaternions (which every atom has used): unit vector and first atom.
+		// The last warp takes them: it has no more pairs than the others.
+		for (int k = TPP - 1 - rank; k < L.ntors; k += TPP) {
+			const int2 ends = L.tors_ends[k];
+			const float3 e0 = ld3(S.xyz + 3 * ends.x), e1 = ld3(S.xyz + 3 * ends.y);
+			float ux = e1.x - e0.x, uy = e1.y - e0.y, uz = e1.z - e0.z;
+			const float l = rnorm3df(ux, uy, uz);
+			ux *= l; uy *= l; uz *= l;
+			S.tq[k] = make_float4(ux, uy, uz, 0.0f);
+			S.tq[L.ntors + k] = make_float4(e0.x, e0.y, e0.z, 0.0f);
+		}
+	}
 
 	// 4. intramolecular pairs (cuda/calcMergeEneGra.cu:418-602)
-	if constexpr (TERMS) e_acc += pair_terms<TPP, GRAD, TERMS>(L, S, rank, tt + 3);
-	else e_acc += pair_terms<TPP, GRAD>(L, S, rank);
+	float e_pair, e_gen = 0.0f;
+	if constexpr (TERMS) e_pair = pair_terms<TPP, GRAD, TERMS>(L, S, rank, tt + 3);
+	else e_pair = pair_terms<TPP, GRAD>(L, S, rank);
 	if (L.ngpairs > 0) {
-		if constexpr (TERMS) e_acc += pair_terms_generic<TPP, GRAD, TERMS>(L, S, rank, tt + 3);
-		else e_acc += pair_terms_generic<TPP, GRAD>(L, S, rank);
+		if constexpr (TERMS) e_gen = pair_terms_generic<TPP, GRAD, TERMS>(L, S, rank, tt + 3);
+		else e_gen = pair_terms_generic<TPP, GRAD>(L, S, rank);
 	}
+	if (GRAD || split) G.sync();   // every pair's forces are in S.f3 (and the upper half's terms in S.gg)
+	if constexpr (kCanSplit) {
+		if (split && rank < TPP / 2) {
+			if (rank < L.natoms) e_acc = reinterpret_cast<const float*>(S.gg)[rank];
+			S.gg[rank] = 0;
+		}
+	}
+	e_acc += e_pair;
+	if (L.ngpairs > 0) e_acc += e_gen;
 	if constexpr (TERMS) {
 		G.template sum_n<8>(tt);
 		if (rank == 0)
 			for (int k = 0; k < 8; k++) terms[k] = tt[k];
 	}
 	if (!GRAD) return G.sum(e_acc);
-	G.sync();   // every pair's forces are in S.f3
 
 	// 5. torque and total force over the ligand atoms (cuda/calcMergeEneGra.cu:608-661);
 	//    the energy rides along as a seventh sum (one cross-warp exchange, not two)
 	// sizes and pointers of the steps below read once (when L lives in shared
 	// memory, the engine's per-task arguments, the stores to S would otherwise
 	// force reloads in every iteration); not held across the pair loop, whose
-	// register peak would spill
-	const int nlig = L.nlig;
+	// register peak would spill.  Every atom's force becomes a float here, once,
+	// for this step and step 6.
+	const int nlig = L.nlig, natoms = L.natoms;
 	const float spacing = L.spacing;
+	float* const ff = reinterpret_cast<float*>(S.f3);
 	float red[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, e_acc};
-	for (int a = rank; a < nlig; a += TPP) {
-		const float3 pa = ld3(S.xyz + 3 * a);
-		float3 r = make_float3((pa.x - gr.mv.x) * spacing, (pa.y - gr.mv.y) * spacing, (pa.z - gr.mv.z) * spacing);
+	for (int a = rank; a < natoms; a += TPP) {
 		const int* fa = S.f3 + 3 * a;
 		float3 f = make_float3(kOneOverTermScale * (float)fa[0], kOneOverTermScale * (float)fa[1], kOneOverTermScale * (float)fa[2]);
-		red[3] += f.x; red[4] += f.y; red[5] += f.z;
-		float3 t = cross3(r, f);
-		red[0] += t.x; red[1] += t.y; red[2] += t.z;
+		ff[3 * a] = f.x; ff[3 * a + 1] = f.y; ff[3 * a + 2] = f.z;
+		if (a < nlig) {
+			const float3 pa = ld3(S.xyz + 3 * a);
+			float3 r = make_float3((pa.x - gr.mv.x) * spacing, (pa.y - gr.mv.y) * spacing, (pa.z - gr.mv.z) * spacing);
+			red[3] += f.x; red[4] += f.y; red[5] += f.z;
+			float3 t = cross3(r, f);
+			red[0] += t.x; red[1] += t.y; red[2] += t.z;
+		}
 	}
 	G.template sum_n<7>(red, true);
 	const float energy = red[6];
-	if (rank < 3 && nlig > 0) {
-		// translation (:676-689) and orientation (:695-815) genes: lane j takes
-		// orientation gene 3 + j (phi, theta, rotation angle) with the same code
-		// on its own angle, and lane 0 also the translation genes; every gene
-		// gets the reference's operations in the reference's order
-		if (rank == 0) {
-			S.gg[0] = quant(red[3] * spacing);
-			S.gg[1] = quant(red[4] * spacing);
-			S.gg[2] = quant(red[5] * spacing);
-		}
+	// translation (:676-689) and orientation (:695-815) genes.  Orientation
+	// gene 3 + j (phi, theta, rotation angle) takes its own target angle, phi by
+	// another formula than the other two, so in groups of several warps phi and
+	// the others sit in different warps; in one warp lane j takes gene 3 + j.
+	// Every gene gets the reference's operations in the reference's order.
+	int j = -1;
+	if constexpr (TPP == 32) j = rank < 3 ? rank : -1;
+	else if constexpr (TPP == 64) j = rank == 0 ? 0 : (rank == 32 || rank == 33 ? rank - 31 : -1);
+	else j = (rank & 31) == 0 && rank < 96 ? rank >> 5 : -1;
+	if (nlig > 0 && rank == (TPP == 128 ? 96 : 0)) {
+		S.gg[0] = quant(red[3] * spacing);
+		S.gg[1] = quant(red[4] * spacing);
+		S.gg[2] = quant(red[5] * spacing);
+	}
+	if (j >= 0 && nlig > 0) {
 		float tl = norm3df(red[0], red[1], red[2]);
 		float oscale = (tl < kInfinitesimalRadian) ? 1.0f : tl * kInvInfinitesimalRadian;
 		// sin/cos of half the infinitesimal rotation (SIN/COS_HALF_INFINITESIMAL_RADIAN,
@@ -823,49 +943,49 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 		// target angle: phi = atan2, theta = 2 pi + sign * acos(z / sin_ang),
 		// rotation = 2 acos(w)
 		float target;
-		if (rank == 0) {
+		if (j == 0) {
 			target = fmod_pi2(atan2f(gr.is_theta_gt_pi * tgt.y, gr.is_theta_gt_pi * tgt.x) + kPiTimes2);
 		} else {
 			const float sin_ang = sqrtf(1.0f - tgt.w * tgt.w);
-			const float ac = fast_acos(rank == 1 ? tgt.z / sin_ang : tgt.w);
-			target = rank == 1 ? kPiTimes2 + gr.is_theta_gt_pi * ac : 2.0f * ac;
+			const float ac = fast_acos(j == 1 ? tgt.z / sin_ang : tgt.w);
+			target = j == 1 ? kPiTimes2 + gr.is_theta_gt_pi * ac : 2.0f * ac;
 		}
-		const float cur = fmod_pi2(kPiTimes2 + g[3 + rank] * kDegToRad);
+		const float cur = fmod_pi2(kPiTimes2 + g[3 + j] * kDegToRad);
 		float v = oscale * (fmod_pi2(target - cur + kPi) - kPi);
 		const float corr = 4.0f * gr.sin_half * gr.sin_half;
-		if (rank == 0) v = v * gr.sin_theta * gr.sin_theta;
-		if (rank <= 1) v = v * corr;
-		S.gg[3 + rank] = quant(v * kDegToRad);
+		if (j == 0) v = v * gr.sin_theta * gr.sin_theta;
+		if (j <= 1) v = v * corr;
+		S.gg[3 + j] = quant(v * kDegToRad);
 	}
 
-	// 6. torsion genes: axis . (r x F) summed over each torsion's rotating atoms (:819-880)
+	// 6. torsion genes: axis . (r x F) summed over each torsion's rotating atoms
+	//    (:819-880).  In groups of several warps the last one, which has the
+	//    least of the above to do, comes first in the order that items are handed
+	//    out, and with 128 threads takes up to three rounds of them alone.
 	const uint32_t* const tor_items = L.tor_items;
-	const int2* const tors_ends = L.tors_ends;
-	const int ntoritems = L.ntoritems, ngenes = L.ngenes;
-	for (int it = rank; it < ntoritems; it += TPP) {
-		uint32_t item = tor_items[it];
-		int k = item >> 8, la = item & 0xFF;
-		int2 ends = tors_ends[k];
-		const float3 e0 = ld3(S.xyz + 3 * ends.x), e1 = ld3(S.xyz + 3 * ends.y), pl = ld3(S.xyz + 3 * la);
-		float rx = e0.x, ry = e0.y, rz = e0.z;
-		float ux = e1.x - rx, uy = e1.y - ry, uz = e1.z - rz;
-		float l = rnorm3df(ux, uy, uz);
-		ux *= l; uy *= l; uz *= l;
-		float3 r = make_float3(pl.x - rx, pl.y - ry, pl.z - rz);
-		const int* fl = S.f3 + 3 * la;
-		float3 f = make_float3(kOneOverTermScale * (float)fl[0], kOneOverTermScale * (float)fl[1], kOneOverTermScale * (float)fl[2]);
+	const int ntoritems = L.ntoritems, ntors = L.ntors;
+	if constexpr (TPP == 32) G.sync();     // the forces of step 5 (larger groups: the barrier in the sum)
+	const bool last_only = TPP == 128 && ntoritems <= 96;
+	const int it0 = last_only ? (rank >= 96 ? rank - 96 : ntoritems) : (rank + 32) & (TPP - 1);
+	for (int it = it0; it < ntoritems; it += last_only ? 32 : TPP) {
+		const uint32_t item = __ldg(tor_items + it);
+		const int k = item >> 8, la = item & 0xFF;
+		const float4 u = S.tq[k], e0 = S.tq[ntors + k];
+		const float3 pl = ld3(S.xyz + 3 * la), f = ld3(ff + 3 * la);
+		float3 r = make_float3(pl.x - e0.x, pl.y - e0.y, pl.z - e0.z);
 		float3 t = cross3(r, f);
-		float on_axis = (ux * t.x + uy * t.y + uz * t.z) * spacing;
+		float on_axis = (u.x * t.x + u.y * t.y + u.z * t.z) * spacing;
 		atomicAdd(&S.gg[6 + k], quant(on_axis * kDegToRad));
 	}
+	const int ngenes = L.ngenes;
 	G.sync();
-	// 7. fixed point -> float, Angstrom/radian scaling of genes >= 3 (:883-899)
+	// 7. fixed point -> float, Angstrom/radian scaling of genes >= 3 (:883-899).
+	//    Gene k is written by the thread that the searches read it in (k mod TPP).
 	const float sc = spacing * spacing * kScAngstromRadian;
 	for (int k = rank; k < ngenes; k += TPP) {
 		float v = kOneOverTermScale * (float)S.gg[k];
 		grad[k] = (k >= 3) ? v * sc : v;
 	}
-	G.sync();
 	return energy;
 }
 

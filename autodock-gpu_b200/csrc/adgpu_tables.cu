@@ -168,7 +168,7 @@ adgpu_status pack_ligand(const adgpu_dockpars& dp, const adgpu_kc_interintra& ii
 	}
 	out.ntoritems = (int)items.size();
 	size_t nchain = 0;
-	for (auto& c : chains) nchain += c.size();
+	for (auto& c : chains) nchain += align_up(c.size(), 4);      // each chain from a multiple of 4 on, read as words
 	if (nchain > 65535) return fail(ADGPU_ERR_LIMIT, "rotation chains too long");
 
 	// layout of the blob
@@ -226,7 +226,8 @@ adgpu_status pack_ligand(const adgpu_dockpars& dp, const adgpu_kc_interintra& ii
 		uint32_t slot = ignore ? 0u : (2u + mt);
 		info[a] = slot | (ignore ? 0x100u : 0u) | (genrot[a] ? 0x200u : 0u) | ((uint32_t)cpos << 16);
 		clen[a] = (uint8_t)chains[a].size();
-		for (uint8_t k : chains[a]) chain[cpos++] = k;
+		for (size_t i = 0; i < chains[a].size(); i++) chain[cpos + i] = chains[a][i];
+		cpos += align_up(chains[a].size(), 4);
 		out.rot_ops += (long)chains[a].size() + (genrot[a] && a < dp.true_ligand_atoms ? 1 : 0);
 		if (ii.atom_types_const[a] >= (uint32_t)dp.num_of_atypes) return fail(ADGPU_ERR_ARG, "atom type out of range");
 	}
