@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256) progress_kernel(const int* evals_runs, in
 	}
 	__syncthreads();
 	if (!s_stop && as.state && g % as.state->as_frequency == 0) {
-		autostop_check(*as.state, as.stats, as.buf_e, as.buf_m, as.energies, (int)g, s_count, s_best);
+		autostop_check(AsBlock{(int)threadIdx.x}, *as.state, as.stats, as.buf_e, as.buf_m, as.energies, (int)g, s_count, s_best);
 		if (threadIdx.x == 0 && as.state->autostopped && tot > as.min_evals) s_stop = 1;
 	}
 	if (threadIdx.x == 0) {
@@ -289,11 +289,25 @@ adgpu_status dock_resident(ApiState& s, int lsmet, uint32_t runs, uint64_t max_e
 {
 	const adgpu_dockpars& dp = s.data.dockpars;
 	memset(&s.pipe.stats, 0, sizeof(s.pipe.stats));
-	if (as_frequency == 0 && s.pipeline && pipeline_applies(dp, runs)) {
+	// (an AutoStop test sums all energies in one thread: with many of them it
+	// would outlast the pipelined loop's idle limit)
+	const bool as_fits = as_frequency == 0 || (uint64_t)runs * (uint64_t)dp.pop_size <= (1u << 18);
+	if (s.pipeline && as_fits && pipeline_applies(dp, runs)) {
 		*autostopped = 0;
 		KArgs base = make_args(s);
-		return dock_pipelined(base, s.pipe, lsmet, s.tpp, runs, max_evals, max_gens, c1, e1, c2, e2,
-		                      final_is_second, generations);
+		PipeAutoStop as;
+		int tpp = s.tpp;
+		if (as_frequency > 0) {
+			as.frequency = as_frequency;
+			as.stopstd = stopstd;
+			as.min_evals = min_as_evals;
+			// the group sizes that the generation-synchronous loop below takes, so
+			// that the sums of a docking with AutoStop are the same in both loops
+			as.ga_tpp = tpp ? tpp : auto_tpp(runs * (uint32_t)dp.pop_size, 0);
+			if (tpp == 0) tpp = auto_tpp(runs * dp.num_of_lsentities, lsmet + 1);
+		}
+		return dock_pipelined(base, s.pipe, lsmet, tpp, runs, max_evals, max_gens, as, c1, e1, c2, e2,
+		                      final_is_second, generations, autostopped);
 	}
 	const uint32_t T = 64;
 	cudaStream_t st;

@@ -6,6 +6,10 @@
 // progress kernel takes the same decision on the device, so a docking with
 // AutoStop needs no per-check copy and no host round trip.
 //
+// Any group of threads with rank, size() and sync() can take it (the progress
+// kernel's block, a pose group of the pipelined loop): what is found in
+// parallel does not depend on how many they are.
+//
 // The statistics are the reference's, operation for operation, with the
 // rounding of its host build: float operations where its operands are float,
 // double where a double literal promotes them, no fused multiply-adds
@@ -71,13 +75,21 @@ __device__ __forceinline__ float as_stddev(const float* a)
 	return __fdiv_rn(__fsqrt_rn(sq), a[2]);
 }
 
-// tabulate_energies (autostop.hpp:83-104) with the whole block: thread t scans
+// A 256-thread block as the group.
+struct AsBlock {
+	int rank;
+	__device__ static constexpr int size() { return 256; }
+	__device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+
+// tabulate_energies (autostop.hpp:83-104) with the whole group: thread t scans
 // a contiguous chunk, the chunks' below-threshold entries are compacted in
 // order into buf_e/buf_m (bin Ntop = none), and thread 0 sums them in order.
-__device__ void as_tabulate(AutoStopState& s, float* a, float* buf_e, uint16_t* buf_m, const float* energies, int n,
+template <class GT>
+__device__ void as_tabulate(const GT& G, AutoStopState& s, float* a, float* buf_e, uint16_t* buf_m, const float* energies, int n,
                             int* s_count, float* s_best)
 {
-	const int T = blockDim.x, t = threadIdx.x;
+	const int T = G.size(), t = G.rank;
 	const int chunk = (n + T - 1) / T, i0 = t * chunk, i1 = min(n, i0 + chunk);
 	const double base = __dsub_rn((double)s.threshold, __dmul_rn(2.0, (double)s.thres_stddev));
 	int cnt = 0;
@@ -89,7 +101,7 @@ __device__ void as_tabulate(AutoStopState& s, float* a, float* buf_e, uint16_t* 
 	}
 	s_count[t] = cnt;
 	s_best[t] = best;
-	__syncthreads();
+	G.sync();
 	if (t == 0) {
 		int run = 0;
 		float b = 1 << 24;
@@ -97,19 +109,25 @@ __device__ void as_tabulate(AutoStopState& s, float* a, float* buf_e, uint16_t* 
 		s_count[T] = run;
 		s.overall_best_energy = b;
 	}
-	__syncthreads();
+	G.sync();
 	int pos = s_count[t];
 	for (int i = i0; i < i1; i++) {
 		const float e = energies[i];
 		if (!(e < s.threshold)) continue;
-		unsigned int m = 0;
-		for (; m < s.Ntop; m++)
-			if ((double)e < __dadd_rn(base, (double)__fmul_rn((float)m, s.delta_energy))) break;
+		// the lowest bin whose upper end is above e (Ntop: none); the ends do not
+		// fall with m, and with a NaN width no bin takes e, so halving finds the
+		// bin that the reference's loop over all of them does
+		unsigned int m = 0, none_below = s.Ntop;
+		while (m < none_below) {
+			const unsigned int h = (m + none_below) / 2;
+			if ((double)e < __dadd_rn(base, (double)__fmul_rn((float)h, s.delta_energy))) none_below = h;
+			else m = h + 1;
+		}
 		buf_e[pos] = e;
 		buf_m[pos] = (uint16_t)m;
 		pos++;
 	}
-	__syncthreads();
+	G.sync();
 	if (t == 0) {
 		const int total = s_count[T];
 		for (int k = 0; k < total; k++) {
@@ -126,11 +144,11 @@ __device__ void as_tabulate(AutoStopState& s, float* a, float* buf_e, uint16_t* 
 			}
 		}
 	}
-	__syncthreads();
+	G.sync();
 }
 
 // set_stats (autostop.hpp:106-129), one thread.
-__device__ void as_set_stats(AutoStopState& s, float* a)
+__device__ inline void as_set_stats(AutoStopState& s, float* a)
 {
 	s.curr_avg = as_average(a);
 	s.curr_std = as_stddev(a);
@@ -156,23 +174,24 @@ __device__ void as_set_stats(AutoStopState& s, float* a)
 	}
 }
 
-// check_if_satisfactory (autostop.hpp:169-222) with the whole block; the
-// result is s.autostopped.  scratch: s_count[blockDim.x + 1], s_best[blockDim.x].
-__device__ void autostop_check(AutoStopState& s, float* a, float* buf_e, uint16_t* buf_m, const float* energies,
+// check_if_satisfactory (autostop.hpp:169-222) with the whole group; the
+// result is s.autostopped.  scratch: s_count[G.size() + 1], s_best[G.size()].
+template <class GT>
+__device__ void autostop_check(const GT& G, AutoStopState& s, float* a, float* buf_e, uint16_t* buf_m, const float* energies,
                                int generation_cnt, int* s_count, float* s_best)
 {
 	const int n = s.num_runs * (int)s.pop_size;
 	const int nstats = (int)(s.pop_size + 1) * 3;
 	const int reps = 1 + 8 * (generation_cnt == 0);
 	for (int count = 0; count < reps; count++) {
-		__syncthreads();
+		G.sync();
 		if (!((double)fabsf(s.curr_avg) > 0.00001)) break;    // uniform: every thread reads the same state
-		__syncthreads();
-		if (threadIdx.x == 0) s.threshold_used = s.threshold;
-		for (int k = threadIdx.x; k < nstats; k += blockDim.x) a[k] = 0.0f;
-		__syncthreads();
-		as_tabulate(s, a, buf_e, buf_m, energies, n, s_count, s_best);
-		if (threadIdx.x == 0) {
+		G.sync();
+		if (G.rank == 0) s.threshold_used = s.threshold;
+		for (int k = G.rank; k < nstats; k += G.size()) a[k] = 0.0f;
+		G.sync();
+		as_tabulate(G, s, a, buf_e, buf_m, energies, n, s_count, s_best);
+		if (G.rank == 0) {
 			if (s.first_time) {
 				s.curr_avg = as_average(a);
 				s.curr_std = as_stddev(a);
@@ -190,8 +209,8 @@ __device__ void autostop_check(AutoStopState& s, float* a, float* buf_e, uint16_
 			}
 		}
 	}
-	__syncthreads();
-	if (threadIdx.x == 0) {
+	G.sync();
+	if (G.rank == 0) {
 		float* r = s.rolling;
 		const unsigned int rc = s.roll_count;
 		const float bn = (float)s.bestN;
@@ -212,7 +231,7 @@ __device__ void autostop_check(AutoStopState& s, float* a, float* buf_e, uint16_
 		if ((as_stddev(a) < s.stopstd) && (generation_cnt >= (int)(4 * s.as_frequency)) && (best_var <= 0.00002f))
 			s.autostopped = 1;
 	}
-	__syncthreads();
+	G.sync();
 }
 
 }  // namespace adgpu

@@ -38,12 +38,22 @@
 // 100 %), so populations, energies and evaluation counts are bit-identical
 // to the generation-synchronous loop; only the PRNG states and the per-entity
 // evaluation counters of the discarded generations differ.
+//
+// AutoStop (the reference's default) is part of check g where as_frequency
+// divides g: the pose group that takes the check runs it on the energies that
+// generation g-1 left, whose buffer no generation overwrites before the check
+// is published, while the other groups work ahead.  Checks are published in
+// order: a later one waits (bounded) for the one before it.  The synchronous
+// loop ends each generation with its longest searches running alone (36-atom
+// ligand, 20 runs, ADADELTA, 64 threads per pose, B200: 90.3 ms a docking; this
+// loop with the same scorer 75.1 ms, the same final populations).
 #include <cuda_runtime.h>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
 
 #include "adgpu_kernels.cuh"
+#include "adgpu_autostop.cuh"
 #include "adgpu_queue.cuh"
 #include "adgpu_pipeline.h"
 
@@ -71,6 +81,7 @@ struct PipeCtl {
 	QueueCtl q;                               // q.alive = runs not retired, q.err, accounting
 	int done;                                 // every run has retired
 	int dec;                                  // checks 0 .. dec-1 have said continue
+	int decided;                              // checks published
 	int stop_gen;                             // -1, or the generations run (the check that said stop)
 	unsigned long long parks;                 // times a run waited for a check before its next generation
 	unsigned long long executed;              // evaluations executed, discarded generations included
@@ -96,6 +107,13 @@ struct PipeArgs {
 	int nbuf;                   // population buffers in use (4 or 8): look-ahead nbuf-1 generations
 	unsigned long long max_evals;
 	unsigned int max_gens;
+	// AutoStop (as_state null: none)
+	AutoStopState* as_state;
+	float* as_stats;            // (pop + 1) * 3
+	float* as_e;                // runs * pop
+	uint16_t* as_m;             // runs * pop
+	unsigned long long as_min_evals;
+	unsigned int as_frequency;
 	int group_bytes;            // shared memory per pose group (header + scratch)
 };
 
@@ -103,7 +121,8 @@ struct PipeHdr {
 	unsigned long long pos;
 	long long t_enter, t_task;       // worker accounting (rank 0; globaltimer ns)
 	unsigned long long busy, ntask, nevals;
-	int task, gen, last, decider, stopped, isum;
+	unsigned long long tot;          // evaluations over all runs at the check this group takes
+	int task, gen, last, decider, stopped, isum, stop;
 };
 constexpr int kPipeHdrBytes = (int)((sizeof(PipeHdr) + 15) / 16 * 16);
 
@@ -190,7 +209,28 @@ __device__ int pipe_take(const PipeArgs& p, int worker, const Group<TPP>& G, int
 	return -1;
 }
 
-template <int TPP, int LSMET>
+// The GA step of a task; GA_TPP < TPP: by the group's first warp.
+template <int TPP, int GA_TPP>
+__device__ __forceinline__ void pipe_ga(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+{
+	if constexpr (GA_TPP == TPP) {
+		ga_block<TPP>(a, pb, b, G, S);
+	} else {
+		static_assert(GA_TPP == 32, "the GA step takes the whole group or its first warp");
+		if (G.rank < 32) {
+			Group<32> W;
+			W.rank = G.rank;
+			W.bar_id = G.bar_id;
+			W.red = G.red;
+			ga_block<32>(a, pb, b, W, S);
+		}
+		G.sync();
+	}
+}
+
+// AS: a docking with AutoStop (its own instantiation: the test's code in the
+// kernel of a docking without it cost that one 4 %).
+template <int TPP, int LSMET, int GA_TPP, bool AS>
 __device__ void pipe_worker(const PipeArgs& p)
 {
 	extern __shared__ __align__(16) char smem[];
@@ -231,7 +271,7 @@ __device__ void pipe_worker(const PipeArgs& p)
 			const KArgs& a = p.ka;
 			const PopBufs pb = p.bufs[g & (p.nbuf - 1)];
 			const uint32_t b = (uint32_t)(run * P + ent);
-			ga_block<TPP>(a, pb, b, G, S);
+			pipe_ga<TPP, GA_TPP>(a, pb, b, G, S);
 			// num_of_lsentities == pop_size: local-search block b is entity b
 			if constexpr (LSMET == LS_SW) sw_block<TPP>(a, pb, b, G, S);
 			else if constexpr (LSMET == LS_AD) gradient_ls_block<TPP, LS_AD>(a, pb, b, G, S);
@@ -274,33 +314,10 @@ __device__ void pipe_worker(const PipeArgs& p)
 				atomicAdd(&p.ctl->acc[slot], (unsigned long long)cum);
 				__threadfence();
 				if (atomicAdd(&p.ctl->fin[slot], 1) + 1 == R) {
-					// every run has completed generation g: check g+1
-					// (check_progress, performdocking.cpp.Cuda:908-942)
-					const unsigned long long tot = atomicExch(&p.ctl->acc[slot], 0ull);
+					// every run has completed generation g: check g+1, taken
+					// below by the whole group
+					H.tot = atomicExch(&p.ctl->acc[slot], 0ull);
 					atomicExch(&p.ctl->fin[slot], 0);
-					const double ev = (double)tot / (double)R / (double)p.max_evals * 100.0;
-					const double gp = (double)(g + 1) / (double)p.max_gens * 100.0;
-					__threadfence();
-					volatile PipeCtl* vc = p.ctl;
-					// a generation run past a stop can still complete everywhere
-					// (its last tasks were taken before the stop was seen)
-					if (vc->stop_gen < 0) {
-						if ((ev > gp ? ev : gp) >= 100.0) {
-							vc->stop_gen = g + 1;
-						} else {
-							// project the stop: generations g+1 .. g+k still to run
-							// at the rate generation g added; start none past g+k+1
-							const unsigned long long target = (unsigned long long)R * p.max_evals;
-							const unsigned long long delta = tot > p.ctl->last_tot ? tot - p.ctl->last_tot : 1ull;
-							const unsigned long long k = (target - tot + delta - 1) / delta;
-							long long lim = (long long)g + (long long)k + 1;
-							if (lim > (long long)p.max_gens - 1) lim = (long long)p.max_gens - 1;
-							if (lim > 0x3fffffff) lim = 0x3fffffff;
-							vc->limit = (int)lim;
-							p.ctl->last_tot = tot;
-							vc->dec = g + 2;
-						}
-					}
 					H.decider = 1;
 				}
 			}
@@ -309,7 +326,54 @@ __device__ void pipe_worker(const PipeArgs& p)
 		}
 		G.sync();
 		if (H.decider) {
+			// (check_progress, performdocking.cpp.Cuda:908-942)
+			volatile PipeCtl* vc = p.ctl;
+			if (G.rank == 0) {
+				// checks are published in order: the one before is at most an
+				// AutoStop test of another group away
+				const long long t0 = global_ns();
+				while (vc->decided != g + 1 && vc->stop_gen < 0 && global_ns() - t0 < p.idle_ns) __nanosleep(200);
+				if (vc->decided != g + 1 && vc->stop_gen < 0) atomicExch(&p.ctl->q.err, 3);
+				const double ev = (double)H.tot / (double)R / (double)p.max_evals * 100.0;
+				const double gp = (double)(g + 1) / (double)p.max_gens * 100.0;
+				// a generation run past a stop can still complete everywhere (its
+				// last tasks were taken before the stop was seen): nothing to decide
+				H.stop = (vc->stop_gen >= 0 || vc->decided != g + 1) ? -1 : ((ev > gp ? ev : gp) >= 100.0);
+			}
 			__threadfence();
+			G.sync();
+			__threadfence();
+			if constexpr (AS) {
+				if (H.stop == 0 && (unsigned int)(g + 1) % p.as_frequency == 0) {
+					// (host/src/performdocking.cpp.Cuda:689-698) on generation g's energies
+					int* s_count = reinterpret_cast<int*>(S.gen);      // TPP + 1, then TPP floats: the gene arrays are free
+					autostop_check(G, *p.as_state, p.as_stats, p.as_e, p.as_m, p.bufs[g & (p.nbuf - 1)].e, g + 1, s_count,
+					               reinterpret_cast<float*>(s_count + TPP + 1));
+					if (G.rank == 0 && p.as_state->autostopped && H.tot > p.as_min_evals) H.stop = 1;
+				}
+			}
+			if (G.rank == 0 && H.stop >= 0) {
+				if (H.stop) {
+					vc->stop_gen = g + 1;
+				} else {
+					// project the stop: generations g+1 .. g+k still to run
+					// at the rate generation g added; start none past g+k+1
+					const unsigned long long tot = H.tot;
+					const unsigned long long target = (unsigned long long)R * p.max_evals;
+					const unsigned long long delta = tot > p.ctl->last_tot ? tot - p.ctl->last_tot : 1ull;
+					const unsigned long long k = (target - tot + delta - 1) / delta;
+					long long lim = (long long)g + (long long)k + 1;
+					if (lim > (long long)p.max_gens - 1) lim = (long long)p.max_gens - 1;
+					if (lim > 0x3fffffff) lim = 0x3fffffff;
+					vc->limit = (int)lim;
+					p.ctl->last_tot = tot;
+					vc->dec = g + 2;
+				}
+				__threadfence();
+				vc->decided = g + 2;
+			}
+			__threadfence();
+			G.sync();
 			for (int r = G.rank; r < R; r += TPP) pipe_try_start(p, r);
 			G.sync();
 		}
@@ -328,16 +392,18 @@ __device__ void pipe_worker(const PipeArgs& p)
 
 constexpr int pipe_min_ctas(int lsmet) { return lsmet == LS_SW ? ADGPU_PIPE_MIN_CTAS_SW : ADGPU_PIPE_MIN_CTAS; }
 
-template <int TPP, int LSMET>
+template <int TPP, int LSMET, int GA_TPP, bool AS>
 __global__ void __launch_bounds__(kPipeThreads, pipe_min_ctas(LSMET)) pipe_kernel(const PipeArgs p)
 {
-	pipe_worker<TPP, LSMET>(p);
+	pipe_worker<TPP, LSMET, GA_TPP, AS>(p);
 }
 
 // Check 0 (before the first generation) and the first generation's GA tasks.
 __global__ void __launch_bounds__(256) pipe_init_kernel(PipeArgs p)
 {
 	__shared__ unsigned long long tot;
+	__shared__ int s_count[257];
+	__shared__ float s_best[256];
 	if (threadIdx.x == 0) tot = 0;
 	__syncthreads();
 	unsigned long long s = 0;
@@ -345,7 +411,11 @@ __global__ void __launch_bounds__(256) pipe_init_kernel(PipeArgs p)
 	atomicAdd(&tot, s);
 	__syncthreads();
 	const double ev = (double)tot / (double)p.runs / (double)p.max_evals * 100.0;
-	const bool stop = ev >= 100.0;     // generations 0 of max_gens >= 1
+	bool stop = ev >= 100.0;           // generations 0 of max_gens >= 1
+	if (!stop && p.as_state) {
+		autostop_check(AsBlock{(int)threadIdx.x}, *p.as_state, p.as_stats, p.as_e, p.as_m, p.bufs[0].e_cur, 0, s_count, s_best);
+		stop = p.as_state->autostopped && tot > p.as_min_evals;
+	}
 	for (int r = threadIdx.x; r < p.runs; r += blockDim.x) {
 		p.started[r] = stop ? kRetired : 1;
 		p.done[r] = 0;
@@ -358,6 +428,7 @@ __global__ void __launch_bounds__(256) pipe_init_kernel(PipeArgs p)
 		c->q.alive = stop ? 0 : p.runs;
 		c->done = stop ? 1 : 0;
 		c->dec = 1;
+		c->decided = 1;
 		c->stop_gen = stop ? 0 : -1;
 		c->q.t_first = ~0ull;
 		c->last_tot = tot;
@@ -387,16 +458,17 @@ __global__ void __launch_bounds__(256) pipe_final_kernel(PipeArgs p, long long* 
 		out[4] = (long long)q.busy_ns; out[5] = (long long)q.tasks;
 		out[6] = q.workers ? (long long)(q.t_last - q.t_first) : 0;
 		out[7] = (long long)p.ctl->parks; out[8] = q.workers; out[9] = (long long)p.ctl->executed;
+		out[10] = p.as_state ? p.as_state->autostopped : 0;
 	}
 }
 
 // Initial check and tasks, the persistent launch, the final accounting; the
 // grid is sized from the kernel's occupancy (persistent: every pose group a
 // worker) and capped by the entities a generation offers.
-template <int TPP, int LSMET>
-static adgpu_status launch_pipe(PipeArgs p, long long* d_out, cudaStream_t st)
+template <int TPP, int LSMET, int GA_TPP, bool AS>
+static adgpu_status launch_pipe_as(PipeArgs p, long long* d_out, cudaStream_t st)
 {
-	auto kfn = pipe_kernel<TPP, LSMET>;
+	auto kfn = pipe_kernel<TPP, LSMET, GA_TPP, AS>;
 	const int gpc = kPipeThreads / TPP;
 	const int bytes = p.group_bytes * gpc;
 	if (bytes > 48 * 1024) ADGPU_CUDA_RET(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "pipeline smem");
@@ -417,6 +489,14 @@ static adgpu_status launch_pipe(PipeArgs p, long long* d_out, cudaStream_t st)
 	pipe_final_kernel<<<1, 256, 0, st>>>(p, d_out);
 	ADGPU_CUDA_RET(cudaGetLastError(), "pipeline final");
 	return ADGPU_OK;
+}
+
+template <int TPP, int LSMET, int GA_TPP = TPP>
+static adgpu_status launch_pipe(const PipeArgs& p, long long* d_out, cudaStream_t st)
+{
+	if (p.as_state) return launch_pipe_as<TPP, LSMET, GA_TPP, true>(p, d_out, st);
+	if constexpr (GA_TPP == TPP) return launch_pipe_as<TPP, LSMET, GA_TPP, false>(p, d_out, st);
+	else return fail(ADGPU_ERR_ARG, "GA group size");
 }
 
 bool pipeline_applies(const adgpu_dockpars& dp, uint32_t runs)
@@ -460,13 +540,15 @@ int pipeline_buffers(int tpp)
 }
 
 adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int tpp, uint32_t runs,
-                            uint64_t max_evals, uint32_t max_gens, float* c1, float* e1, float* c2, float* e2,
-                            int* final_is_second, uint32_t* generations)
+                            uint64_t max_evals, uint32_t max_gens, const PipeAutoStop& as, float* c1, float* e1,
+                            float* c2, float* e2, int* final_is_second, uint32_t* generations, int* autostopped)
 {
 	const adgpu_dockpars& dp = base.dp;
 	if (!pipeline_applies(dp, runs)) return fail(ADGPU_ERR_ARG, "pipelined docking needs a 100 % local-search rate");
 	if (tpp == 0) tpp = pipeline_default_tpp(lsmet, (long)runs * dp.pop_size);
 	if (tpp != 32 && tpp != 64 && tpp != 128) return fail(ADGPU_ERR_ARG, "threads per pose must be 32, 64 or 128");
+	const int ga_tpp = as.frequency ? as.ga_tpp : tpp;
+	if (ga_tpp != tpp && (ga_tpp != 32 || tpp != 64)) return fail(ADGPU_ERR_ARG, "GA group size");
 	const int P = dp.pop_size;
 	const size_t n = (size_t)runs * P;
 	const int nbuf = pipeline_buffers(tpp);
@@ -478,7 +560,10 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 	const size_t o_slots = o_e + e_b, slots_b = al((size_t)runs * 8);
 	const size_t o_runs = o_slots + slots_b, runs_b = al((size_t)runs * 4) * 4 + al((size_t)runs * kPipeBufs * 4);
 	const size_t o_ctl = o_runs + runs_b, ctl_b = al(sizeof(PipeCtl)) + 256;
-	const size_t total = o_ctl + ctl_b;
+	// AutoStop: state, statistics, the energies below the threshold and their bins
+	const size_t o_as = o_ctl + ctl_b, as_stats_b = al(autostop_stats_floats(P) * 4);
+	const size_t as_b = as.frequency ? al(sizeof(AutoStopState)) + as_stats_b + al(n * 4) + al(n * 2) : 0;
+	const size_t total = o_as + as_b;
 	if (sc.bytes < total) {
 		if (sc.mem) cudaFree(sc.mem);
 		sc.mem = nullptr; sc.bytes = 0;
@@ -521,6 +606,18 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 	// second buffer: genes past num_of_genes are never written
 	ADGPU_CUDA_RET(cudaMemsetAsync(m + o_conf, 0, conf_b + e_b, st), "pipeline buffers");
 	ADGPU_CUDA_RET(cudaMemsetAsync(p.ctl, 0, sizeof(PipeCtl), st), "pipeline control");
+	AutoStopState as_init;
+	if (as.frequency) {
+		char* b = m + o_as;
+		p.as_state = reinterpret_cast<AutoStopState*>(b); b += al(sizeof(AutoStopState));
+		p.as_stats = reinterpret_cast<float*>(b); b += as_stats_b;
+		p.as_e = reinterpret_cast<float*>(b); b += al(n * 4);
+		p.as_m = reinterpret_cast<uint16_t*>(b);
+		p.as_frequency = as.frequency;
+		p.as_min_evals = as.min_evals;
+		autostop_init(as_init, P, (int)runs, as.stopstd, as.frequency);
+		ADGPU_CUDA_RET(cudaMemcpyAsync(p.as_state, &as_init, sizeof(as_init), cudaMemcpyHostToDevice, st), "autostop init");
+	}
 	adgpu_status rc = ADGPU_OK;
 #define ADGPU_PIPE_LSMET(T) \
 	switch (lsmet) { \
@@ -531,12 +628,18 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 	}
 	switch (tpp) {
 	case 32: ADGPU_PIPE_LSMET(32) break;
-	case 64: ADGPU_PIPE_LSMET(64) break;
+	case 64:
+		// (the other searches take 64 threads only where the GA does)
+		if (ga_tpp == 32 && lsmet == 0) rc = launch_pipe<64, LS_SW, 32>(p, d_out, st);
+		else if (ga_tpp == 32 && lsmet == 1) rc = launch_pipe<64, LS_AD, 32>(p, d_out, st);
+		else if (ga_tpp == 32) rc = fail(ADGPU_ERR_ARG, "GA group size");
+		else ADGPU_PIPE_LSMET(64)
+		break;
 	default: ADGPU_PIPE_LSMET(128) break;
 	}
 #undef ADGPU_PIPE_LSMET
 	if (rc != ADGPU_OK) return rc;
-	ADGPU_CUDA_RET(cudaMemcpyAsync(sc.host_out, d_out, 10 * sizeof(long long), cudaMemcpyDeviceToHost, st), "pipeline readback");
+	ADGPU_CUDA_RET(cudaMemcpyAsync(sc.host_out, d_out, 11 * sizeof(long long), cudaMemcpyDeviceToHost, st), "pipeline readback");
 	ADGPU_CUDA_RET(cudaStreamSynchronize(st), "pipeline docking");
 	const long long* o = sc.host_out;
 	const int G = (int)o[0], alive = (int)o[1], err = (int)o[2];
@@ -558,6 +661,7 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 		                                ", runs still active " + std::to_string(alive) + ")");
 	*generations = (uint32_t)G;
 	*final_is_second = G & 1;
+	*autostopped = (int)o[10];
 	const int fb = G & (nbuf - 1);
 	if (fb >= 2) {
 		// the final population sits in a library buffer: copy it to the

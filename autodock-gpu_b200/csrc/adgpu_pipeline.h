@@ -23,6 +23,14 @@ struct PipeScratch {
 	adgpu_dock_stats stats{};        // accounting of the last call
 };
 
+// AutoStop of a pipelined docking; frequency 0: none.
+struct PipeAutoStop {
+	uint32_t frequency = 0;          // generations between checks
+	float stopstd = 0.0f;
+	unsigned long long min_evals = 0;
+	int ga_tpp = 0;                  // threads per pose of the GA step (the searches' own, or 32 where they take 64)
+};
+
 // Whether the pipelined loop can dock these settings with the reference's
 // results: every run's local searches must draw only on its own PRNG states,
 // which holds when the local-search rate is 100 % (num_of_lsentities ==
@@ -30,9 +38,9 @@ struct PipeScratch {
 bool pipeline_applies(const adgpu_dockpars& dp, uint32_t runs);
 
 // The generation loop of docking_with_gpu as one persistent launch; the
-// arguments and results are those of adgpu_dock_resident.  tpp 0: default.
+// arguments and results are those of adgpu_dock_resident_autostop.  tpp 0: default.
 adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int tpp, uint32_t runs,
-                            uint64_t max_evals, uint32_t max_gens, float* c1, float* e1, float* c2, float* e2,
-                            int* final_is_second, uint32_t* generations);
+                            uint64_t max_evals, uint32_t max_gens, const PipeAutoStop& as, float* c1, float* e1,
+                            float* c2, float* e2, int* final_is_second, uint32_t* generations, int* autostopped);
 
 }  // namespace adgpu
