@@ -84,20 +84,22 @@ struct AsBlock {
 
 // tabulate_energies (autostop.hpp:83-104) with the whole group: thread t scans
 // a contiguous chunk, the chunks' below-threshold entries are compacted in
-// order into buf_e/buf_m (bin Ntop = none), and thread 0 sums them in order.
+// order into buf_e/buf_m (bin Ntop = none) and summed in order.
 template <class GT>
 __device__ void as_tabulate(const GT& G, AutoStopState& s, float* a, float* buf_e, uint16_t* buf_m, const float* energies, int n,
                             int* s_count, float* s_best)
 {
 	const int T = G.size(), t = G.rank;
 	const int chunk = (n + T - 1) / T, i0 = t * chunk, i1 = min(n, i0 + chunk);
-	const double base = __dsub_rn((double)s.threshold, __dmul_rn(2.0, (double)s.thres_stddev));
+	const float threshold = s.threshold, delta = s.delta_energy;
+	const unsigned int Ntop = s.Ntop;
+	const double base = __dsub_rn((double)threshold, __dmul_rn(2.0, (double)s.thres_stddev));
 	int cnt = 0;
 	float best = 1 << 24;
 	for (int i = i0; i < i1; i++) {
 		const float e = energies[i];
 		if (e < best) best = e;
-		cnt += e < s.threshold;
+		cnt += e < threshold;
 	}
 	s_count[t] = cnt;
 	s_best[t] = best;
@@ -113,30 +115,42 @@ __device__ void as_tabulate(const GT& G, AutoStopState& s, float* a, float* buf_
 	int pos = s_count[t];
 	for (int i = i0; i < i1; i++) {
 		const float e = energies[i];
-		if (!(e < s.threshold)) continue;
+		if (!(e < threshold)) continue;
 		// the lowest bin whose upper end is above e (Ntop: none); the ends do not
 		// fall with m, and with a NaN width no bin takes e, so halving finds the
 		// bin that the reference's loop over all of them does
-		unsigned int m = 0, none_below = s.Ntop;
+		unsigned int m = 0, none_below = Ntop;
 		while (m < none_below) {
 			const unsigned int h = (m + none_below) / 2;
-			if ((double)e < __dadd_rn(base, (double)__fmul_rn((float)h, s.delta_energy))) none_below = h;
+			if ((double)e < __dadd_rn(base, (double)__fmul_rn((float)h, delta))) none_below = h;
 			else m = h + 1;
 		}
 		buf_e[pos] = e;
 		buf_m[pos] = (uint16_t)m;
 		pos++;
 	}
+	// The sums in the reference's order.  Each bin has one thread, which takes
+	// the bin's energies in order, and thread 0 takes all of them; the group
+	// stages T energies at a time.  (By one thread alone, whose every addition
+	// waits for the bin's memory, 3,000 energies took longer than a third of a
+	// generation.)
 	G.sync();
-	if (t == 0) {
-		const int total = s_count[T];
-		for (int k = 0; k < total; k++) {
-			const float e = buf_e[k];
-			a[0] = __fadd_rn(a[0], e);
-			a[1] = __fadd_rn(a[1], __fmul_rn(e, e));
-			a[2] = (float)__dadd_rn((double)a[2], 1.0);
-			const unsigned int m = buf_m[k];
-			if (m < s.Ntop) {
+	const int total = s_count[T];
+	float sum = 0.0f, sq = 0.0f, num = 0.0f;
+	for (int i0 = 0; i0 < total; i0 += T) {
+		G.sync();
+		if (i0 + t < total) { s_best[t] = buf_e[i0 + t]; s_count[t] = (int)buf_m[i0 + t]; }
+		G.sync();
+		const int k1 = min(T, total - i0);
+		for (int k = 0; k < k1; k++) {
+			const float e = s_best[k];
+			const unsigned int m = (unsigned int)s_count[k];
+			if (t == 0) {
+				sum = __fadd_rn(sum, e);
+				sq = __fadd_rn(sq, __fmul_rn(e, e));
+				num = (float)__dadd_rn((double)num, 1.0);
+			}
+			if (m < Ntop && m % (unsigned int)T == (unsigned int)t) {
 				float* b = a + 3 * (m + 1);
 				b[0] = __fadd_rn(b[0], e);
 				b[1] = __fadd_rn(b[1], __fmul_rn(e, e));
@@ -144,6 +158,7 @@ __device__ void as_tabulate(const GT& G, AutoStopState& s, float* a, float* buf_
 			}
 		}
 	}
+	if (t == 0) { a[0] = sum; a[1] = sq; a[2] = num; }
 	G.sync();
 }
 
