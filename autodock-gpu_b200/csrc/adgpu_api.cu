@@ -47,14 +47,14 @@ adgpu_status cuda_fail(cudaError_t e, const char* what)
 // ---------------------------------------------------------------------------
 constexpr int lga_min_ctas(int kind) { return kind >= 2 && kind <= 4 ? ADGPU_MIN_CTAS_GRAD : ADGPU_MIN_CTAS; }
 
-template <int TPP, int KIND>
+template <int TPP, int KIND, int SUMS>
 __global__ void __launch_bounds__(128, lga_min_ctas(KIND)) lga_kernel(KArgs a, float* grads)
 {
 	if (a.stop_flag && *a.stop_flag) return;
 	int gid, ngroups;
 	Group<TPP> G;
 	GroupSmem S;
-	group_of<TPP>(a, gid, ngroups, G, S);
+	group_of<TPP, SUMS>(a, gid, ngroups, G, S);
 	// Local searches run for a data-dependent number of iterations, so pose
 	// groups take the next block from a counter instead of a fixed stride.
 	auto next = [&](uint32_t cur) -> uint32_t {
@@ -72,14 +72,14 @@ __global__ void __launch_bounds__(128, lga_min_ctas(KIND)) lga_kernel(KArgs a, f
 		return b;
 	};
 	for (uint32_t b = gid; b < a.nblocks; b = next(b)) {
-		if constexpr (KIND == 0) ga_block<TPP>(a, b, G, S);
-		else if constexpr (KIND == 1) sw_block<TPP>(a, b, G, S);
-		else if constexpr (KIND == 2) gradient_ls_block<TPP, LS_AD>(a, b, G, S);
-		else if constexpr (KIND == 3) gradient_ls_block<TPP, LS_ADAM>(a, b, G, S);
-		else if constexpr (KIND == 4) fire_block<TPP>(a, b, G, S);
-		else if constexpr (KIND == 5) initpop_block<TPP>(a, b, G, S);
-		else if constexpr (KIND == 6) score_block<TPP, false>(a, b, G, S, grads);
-		else if constexpr (KIND == 7) score_block<TPP, true>(a, b, G, S, grads);
+		if constexpr (KIND == 0) ga_block<TPP, SUMS>(a, b, G, S);
+		else if constexpr (KIND == 1) sw_block<TPP, SUMS>(a, b, G, S);
+		else if constexpr (KIND == 2) gradient_ls_block<TPP, LS_AD, SUMS>(a, b, G, S);
+		else if constexpr (KIND == 3) gradient_ls_block<TPP, LS_ADAM, SUMS>(a, b, G, S);
+		else if constexpr (KIND == 4) fire_block<TPP, SUMS>(a, b, G, S);
+		else if constexpr (KIND == 5) initpop_block<TPP, SUMS>(a, b, G, S);
+		else if constexpr (KIND == 6) score_block<TPP, false, SUMS>(a, b, G, S, grads);
+		else if constexpr (KIND == 7) score_block<TPP, true, SUMS>(a, b, G, S, grads);
 		else if constexpr (KIND == 8) score_terms_block<TPP>(a, b, G, S, grads);
 	}
 }
@@ -173,13 +173,13 @@ __global__ void relayout_grid_kernel(const float* __restrict__ ref, float* __res
 // ---------------------------------------------------------------------------
 int g_num_sms = 0;
 
-template <int TPP, int KIND>
+template <int TPP, int KIND, int SUMS = TPP>
 adgpu_status launch_lga(const KArgs& a, float* grads, cudaStream_t stream, int cta_threads)
 {
 	if (a.nblocks == 0) return ADGPU_OK;
 	const int gpc = cta_threads / TPP;
-	const int bytes = group_smem_bytes(a.L.natoms, a.L.ntors, (int)a.ref_threads, TPP) * gpc;
-	auto kfn = lga_kernel<TPP, KIND>;
+	const int bytes = group_smem_bytes(a.L.natoms, a.L.ntors, (int)a.ref_threads, TPP, ep_records(a.L, TPP, SUMS)) * gpc;
+	auto kfn = lga_kernel<TPP, KIND, SUMS>;
 	if (bytes > 48 * 1024) ADGPU_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "smem attribute");
 	static int carveout = -2;           // per instantiation: the last preference set
 	const int pct = smem_carveout_pct(bytes, lga_min_ctas(KIND));
@@ -215,20 +215,31 @@ adgpu_status launch_lga(const KArgs& a, float* grads, cudaStream_t stream, int c
 // threads (6 CTAs of 128 threads per SM), else 32.
 static int auto_tpp(uint32_t n, int kind)
 {
-	if (kind == 1 || kind == 2) return 64;
 	if (g_num_sms == 0) {
 		int dev = 0;
 		if (cudaGetDevice(&dev) != cudaSuccess ||
-		    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 32;
+		    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+			return kind == 1 || kind == 2 ? 64 : 32;
 	}
+	if (kind == 1 || kind == 2) return 64;
 	const long groups32 = (long)g_num_sms * ADGPU_MIN_CTAS * 4;
 	return (long)n * 2 <= groups32 ? 64 : 32;
 }
 
+// Pose groups of 128 threads per SM up to which they beat twice as many of 64.
+constexpr long kShareGroupsPerSm = 4;
+
 template <int KIND>
 adgpu_status launch_kind(const KArgs& a, float* grads, cudaStream_t stream, int tpp)
 {
-	if (tpp == 0) tpp = auto_tpp(a.nblocks, KIND);
+	if (tpp == 0) {
+		tpp = auto_tpp(a.nblocks, KIND);
+		// a launch that leaves SMs short of work takes 128 threads per pose
+		// with the sums of 64, so its results stay those of 64
+		if constexpr (KIND != 8)
+			if (tpp == 64 && shares_sums(a.L) && (long)a.nblocks <= kShareGroupsPerSm * (long)g_num_sms)
+				return launch_lga<128, KIND, 64>(a, grads, stream, 128);
+	}
 	switch (tpp) {
 	case 32: return launch_lga<32, KIND>(a, grads, stream, 128);
 	case 64: return launch_lga<64, KIND>(a, grads, stream, 128);
@@ -304,7 +315,10 @@ adgpu_status dock_resident(ApiState& s, int lsmet, uint32_t runs, uint64_t max_e
 			// the group sizes that the generation-synchronous loop below takes, so
 			// that the sums of a docking with AutoStop are the same in both loops
 			as.ga_tpp = tpp ? tpp : auto_tpp(runs * (uint32_t)dp.pop_size, 0);
-			if (tpp == 0) tpp = auto_tpp(runs * dp.num_of_lsentities, lsmet + 1);
+			if (tpp == 0) {
+				tpp = auto_tpp(runs * dp.num_of_lsentities, lsmet + 1);
+				as.share = tpp == 64 && shares_sums(base.L) && pipeline_default_tpp(lsmet, (long)runs * dp.pop_size) == 128;
+			}
 		}
 		return dock_pipelined(base, s.pipe, lsmet, tpp, runs, max_evals, max_gens, as, c1, e1, c2, e2,
 		                      final_is_second, generations, autostopped);

@@ -339,6 +339,7 @@ struct PoseSmem {
 	float* xyz;
 	int* f3;
 	float4* tq;
+	float2* ep;        // shared sums (shares_sums): the pair records' energies
 	float2* gsc;       // sin/cos of theta, phi and half the rotation angle
 	int* gg;
 };
@@ -362,6 +363,7 @@ __device__ __forceinline__ PoseSmem carve_pose(char* base, int natoms, int ntors
 	f += 3 * n4;
 	s.f3 = reinterpret_cast<int*>(f);
 	s.gg = s.f3 + 3 * n4;
+	s.ep = nullptr;
 	return s;
 }
 
@@ -444,12 +446,22 @@ __device__ __forceinline__ void pair_force(int* f3, uint32_t i, uint32_t j, floa
 // wrap, and every atom's forces start at minus the sum of its offsets over
 // the ligand's records (L.f3_bias, from the tables), so they end exact.
 __device__ __forceinline__ float clamp_term(float v) { return fminf(kMaxTerm, fmaxf(-kMaxTerm, v)); }
-__device__ __forceinline__ void couple_force(unsigned* f3, uint32_t c, uint32_t i, uint32_t j, float2 gx, float2 gy, float2 gz)
+// pg: the pairs' forces along their axes, unscaled.  A component is at most
+// that times 1024 (and rounding), so a warp whose pairs are all below 7.999 in
+// size needs no clamp: most steps of a search, 12 instructions each (docking
+// of 100 runs, ADADELTA, B200: 126.6 -> 125.6 ms).  NaN and infinity fail the
+// test.
+__device__ __forceinline__ void couple_force(unsigned* f3, uint32_t c, uint32_t i, uint32_t j, float2 gx, float2 gy, float2 gz,
+                                             float2 pg)
 {
 	const float2 mg = f2s(kRoundMagic);
-	const float2 rx = f2add(f2(clamp_term(gx.x), clamp_term(gx.y)), mg);
-	const float2 ry = f2add(f2(clamp_term(gy.x), clamp_term(gy.y)), mg);
-	const float2 rz = f2add(f2(clamp_term(gz.x), clamp_term(gz.y)), mg);
+	const bool small = fabsf(pg.x) < 7.999f && fabsf(pg.y) < 7.999f;
+	if (!__all_sync(0xffffffffu, small)) {
+		gx = f2(clamp_term(gx.x), clamp_term(gx.y));
+		gy = f2(clamp_term(gy.x), clamp_term(gy.y));
+		gz = f2(clamp_term(gz.x), clamp_term(gz.y));
+	}
+	const float2 rx = f2add(gx, mg), ry = f2add(gy, mg), rz = f2add(gz, mg);
 	const unsigned ax = __float_as_uint(rx.x), ay = __float_as_uint(ry.x), az = __float_as_uint(rz.x);
 	const unsigned bx = __float_as_uint(rx.y), by = __float_as_uint(ry.y), bz = __float_as_uint(rz.y);
 	unsigned* fc = f3 + 3 * c;
@@ -472,7 +484,8 @@ __device__ __forceinline__ void couple_force(unsigned* f3, uint32_t c, uint32_t 
 // With COUPLED (the host's tables, L.coupled) the two pairs of a record share
 // their first atom: one position load and one set of atomics for it.  CGG0:
 // the ligand has CG-G0 pairs (flexible rings).
-template <int TPP, bool GRAD, bool TERMS, bool COUPLED, bool CGG0>
+// EP: each record's energies go to S.ep instead (pair_sum).
+template <int TPP, bool GRAD, bool TERMS, bool COUPLED, bool CGG0, bool EP = false>
 __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, int rank, float* tsum)
 {
 	// loop invariants read once: when L lives in shared memory (the engine's
@@ -581,14 +594,15 @@ __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, i
 				pg = f2fma(f2s(-1.0f), f2mul(in20, ge), pg);
 			}
 		}
-		esum = f2add(esum, e);
+		if constexpr (EP) S.ep[d] = e;
+		else esum = f2add(esum, e);
 		if (GRAD) {
 			// fixed-point forces; the 1024 scale folded into gdd (a power of two:
 			// the same rounding as quant(sub * gdd))
 			const float2 gdd = f2mul(pg, f2mul(inv_dist, f2s(-kTermScale)));
 			const float2 gx = f2mul(sx, gdd), gy = f2mul(sy, gdd), gz = f2mul(sz, gdd);
 			if constexpr (COUPLED) {
-				couple_force(reinterpret_cast<unsigned*>(f3), a1, a2, b2, gx, gy, gz);
+				couple_force(reinterpret_cast<unsigned*>(f3), a1, a2, b2, gx, gy, gz, pg);
 			} else {
 				pair_force(f3, a1, a2, gx.x, gy.x, gz.x);
 				pair_force(f3, b1, b2, gx.y, gy.y, gz.y);
@@ -601,6 +615,15 @@ __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, i
 		tsum[2] += t_ds.x + t_ds.y;
 		tsum[3] += t_cg.x + t_cg.y;
 	}
+	return esum.x + esum.y;
+}
+
+// The sum of pair_loop<SUMS> for thread rank < SUMS, from S.ep.
+template <int SUMS>
+__device__ __forceinline__ float pair_sum(const LigDev& L, const PoseSmem& S, int rank)
+{
+	float2 esum = f2s(0.0f);
+	for (int d = rank; d < L.npairs2; d += SUMS) esum = f2add(esum, S.ep[d]);
 	return esum.x + esum.y;
 }
 
@@ -663,6 +686,14 @@ __device__ __forceinline__ float pair_terms_generic(const LigDev& L, const PoseS
 	return esum;
 }
 
+// Whether a group of 128 threads can take the sums of one of 64 (score_pose's
+// SUMS): each thread of the lower half then has at most one atom, and the
+// records' energies, added up by the lower half, take at most 8 KB.
+__host__ __device__ inline bool shares_sums(const LigDev& L)
+{
+	return L.coupled && L.ngpairs == 0 && L.natoms <= 64 && L.npairs2 <= 1024;
+}
+
 // ---- the scorer -----------------------------------------------------------------------
 // Scores genotype g (shared memory, read-only here).  Returns the energy (same
 // value in every thread of the group).  With GRAD, writes dE/dgene to
@@ -691,14 +722,20 @@ __device__ __forceinline__ float pair_terms_generic(const LigDev& L, const PoseS
 // early loads lost 2 % at 64 threads and 32).  Every float is computed by the same operations in the same
 // order whatever the group does in parallel, and each thread adds up the same
 // terms: results do not depend on it.
-template <int TPP, bool GRAD, bool REF_GRID = false, bool TERMS = false>
+//
+// SUMS: the group size whose sums are taken.  Float sums depend on how a pose
+// is dealt out to threads, and a search of hundreds of steps on every bit of
+// them; SUMS 64 with 128 threads (shares_sums) gives what 64 threads give, in
+// the shorter time of 128.
+template <int TPP, bool GRAD, bool REF_GRID = false, bool TERMS = false, int SUMS = TPP>
 __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float* __restrict__ grad,
                            const PoseSmem& S, const Group<TPP>& G, float* terms = nullptr)
 {
 	const int rank = G.rank;
 	// the upper half takes the lower half's intermolecular terms
 	constexpr bool kCanSplit = TPP == 128 && !TERMS && !REF_GRID;
-	const bool split = kCanSplit && L.natoms <= TPP / 2;
+	static_assert(SUMS == TPP || (SUMS == 64 && kCanSplit), "sums of another group size");
+	const bool split = kCanSplit && (SUMS != TPP || L.natoms <= TPP / 2);
 
 	// 0. this thread's first atom (with split, the upper half's: its partner's)
 	struct AtomIn { float4 r; uint32_t info, chain; int len; };
@@ -868,7 +905,10 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 
 	// 4. intramolecular pairs (cuda/calcMergeEneGra.cu:418-602)
 	float e_pair, e_gen = 0.0f;
-	if constexpr (TERMS) e_pair = pair_terms<TPP, GRAD, TERMS>(L, S, rank, tt + 3);
+	if constexpr (SUMS != TPP) {
+		e_pair = L.cgg0 ? pair_loop<TPP, GRAD, false, true, true, true>(L, S, rank, nullptr)
+		                : pair_loop<TPP, GRAD, false, true, false, true>(L, S, rank, nullptr);
+	} else if constexpr (TERMS) e_pair = pair_terms<TPP, GRAD, TERMS>(L, S, rank, tt + 3);
 	else e_pair = pair_terms<TPP, GRAD>(L, S, rank);
 	if (L.ngpairs > 0) {
 		if constexpr (TERMS) e_gen = pair_terms_generic<TPP, GRAD, TERMS>(L, S, rank, tt + 3);
@@ -879,6 +919,7 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 		if (split && rank < TPP / 2) {
 			if (rank < L.natoms) e_acc = reinterpret_cast<const float*>(S.gg)[rank];
 			S.gg[rank] = 0;
+			if constexpr (SUMS != TPP) e_pair = pair_sum<SUMS>(L, S, rank);
 		}
 	}
 	e_acc += e_pair;

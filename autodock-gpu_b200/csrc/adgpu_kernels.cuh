@@ -46,6 +46,10 @@ struct PopBufs {
 
 __device__ __forceinline__ PopBufs bufs_of(const KArgs& a) { return PopBufs{a.conf_cur, a.e_cur, a.conf, a.e}; }
 
+// Pair records whose energies a group of tpp threads with the sums of `sums`
+// threads keeps in shared memory.
+__host__ __device__ inline int ep_records(const LigDev& L, int tpp, int sums) { return sums != tpp ? L.npairs2 : 0; }
+
 // Per-group scratch carved from dynamic shared memory.
 struct GroupSmem {
 	PoseSmem pose;
@@ -71,9 +75,10 @@ inline int smem_carveout_pct(int bytes, int ctas)
 	return (int)(pct > 100 ? 100 : pct);
 }
 
-__host__ __device__ inline int group_smem_bytes(int natoms, int ntors, int ref_threads, int tpp)
+// ep: pair records whose energies the group keeps (ep_records), else 0
+__host__ __device__ inline int group_smem_bytes(int natoms, int ntors, int ref_threads, int tpp, int ep = 0)
 {
-	int b = pose_smem_bytes(natoms, ntors);
+	int b = pose_smem_bytes(natoms, ntors) + ep * 8;
 	b += 8 * 64 * 4;                       // gene arrays
 	b += ((ref_threads + 3) & ~3) * 4;     // PRNG states
 	b += (tpp / 32) * 8 * 4;               // reduction scratch
@@ -81,11 +86,13 @@ __host__ __device__ inline int group_smem_bytes(int natoms, int ntors, int ref_t
 	return (b + 15) & ~15;
 }
 
-__device__ __forceinline__ GroupSmem carve_group(char* base, int natoms, int ntors, int ref_threads, int tpp)
+__device__ __forceinline__ GroupSmem carve_group(char* base, int natoms, int ntors, int ref_threads, int tpp, int ep = 0)
 {
 	GroupSmem s;
 	s.pose = carve_pose(base, natoms, ntors);
-	float* f = reinterpret_cast<float*>(base + pose_smem_bytes(natoms, ntors));
+	base += pose_smem_bytes(natoms, ntors);
+	s.pose.ep = reinterpret_cast<float2*>(base);
+	float* f = reinterpret_cast<float*>(base + ep * 8);
 	s.gen = f; s.best = f + 64; s.grad = f + 128; s.s1 = f + 192; s.s2 = f + 256; s.s3 = f + 320; s.s4 = f + 384; s.s5 = f + 448;
 	f += 512;
 	s.st = reinterpret_cast<uint32_t*>(f);
@@ -98,7 +105,7 @@ __device__ __forceinline__ GroupSmem carve_group(char* base, int natoms, int nto
 }
 
 // The group of this thread and its scratch.
-template <int TPP>
+template <int TPP, int SUMS = TPP>
 __device__ __forceinline__ void group_of(const KArgs& a, int& gid, int& ngroups, Group<TPP>& G, GroupSmem& S)
 {
 	extern __shared__ __align__(16) char smem[];
@@ -106,8 +113,8 @@ __device__ __forceinline__ void group_of(const KArgs& a, int& gid, int& ngroups,
 	const int local = threadIdx.x / TPP;
 	gid = blockIdx.x * gpc + local;
 	ngroups = gridDim.x * gpc;
-	const int bytes = group_smem_bytes(a.L.natoms, a.L.ntors, (int)a.ref_threads, TPP);
-	S = carve_group(smem + local * bytes, a.L.natoms, a.L.ntors, (int)a.ref_threads, TPP);
+	const int bytes = group_smem_bytes(a.L.natoms, a.L.ntors, (int)a.ref_threads, TPP, ep_records(a.L, TPP, SUMS));
+	S = carve_group(smem + local * bytes, a.L.natoms, a.L.ntors, (int)a.ref_threads, TPP, ep_records(a.L, TPP, SUMS));
 	G.rank = threadIdx.x % TPP;
 	G.bar_id = 1 + local;
 	G.red = S.red;
@@ -138,7 +145,7 @@ __device__ __forceinline__ int ls_entity(const KArgs& a, uint32_t b, const Group
 // success/fail step-size proxy falls to 0.01 or after max_num_of_iters.
 // ADAM (cuda/kernel_adam.cu:55-396): bias-corrected, always max_num_of_iters.
 // ---------------------------------------------------------------------------
-template <int TPP, int METHOD>
+template <int TPP, int METHOD, int SUMS = TPP>
 __device__ void gradient_ls_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
 {
 	const int P = a.dp.pop_size, NG = a.dp.num_of_genes;
@@ -165,7 +172,7 @@ __device__ void gradient_ls_block(const KArgs& a, const PopBufs& pb, uint32_t b,
 			b1r = 1.0f - powf(a.dp.adam_beta1, t);
 			b2r = 1.0f - powf(a.dp.adam_beta2, t);
 		}
-		const float energy = score_pose<TPP, true>(a.L, S.gen, S.grad, S.pose, G);
+		const float energy = score_pose<TPP, true, false, false, SUMS>(a.L, S.gen, S.grad, S.pose, G);
 		float b1p = 0.f, b2p = 0.f;
 		if (METHOD == LS_ADAM) {
 			b1p = __shfl_sync(0xffffffffu, b1r, (int)(it & 31u));
@@ -216,7 +223,7 @@ __device__ void gradient_ls_block(const KArgs& a, const PopBufs& pb, uint32_t b,
 // FIRE (device/kernel_fire.cl:76-895): N_min 5, f_inc 1.2, f_dec 0.8,
 // alpha0 0.2, f_alpha 0.99, dt_max 10, dt0 = dt_max/3, stop at dt < 1e-6.
 // ---------------------------------------------------------------------------
-template <int TPP>
+template <int TPP, int SUMS = TPP>
 __device__ void fire_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
 {
 	const float DT_INC = 1.2f, DT_DEC = 0.8f, ALPHA_START = 0.2f, ALPHA_DEC = 0.99f, DT_MAX = 10.0f, DT_MIN = 1e-6f;
@@ -231,7 +238,7 @@ __device__ void fire_block(const KArgs& a, const PopBufs& pb, uint32_t b, const 
 	G.sync();
 	float energy = pb.e[idx];
 	// initial gradient (the OpenCL kernel's gradient-only call, taken from the merged scorer)
-	score_pose<TPP, true>(a.L, gen, grad, S.pose, G);
+	score_pose<TPP, true, false, false, SUMS>(a.L, gen, grad, S.pose, G);
 	auto sumsq = [&](const float* v) {
 		float s = 0.f;
 		for (int k = G.rank; k < NG; k += TPP) s += v[k] * v[k];
@@ -246,7 +253,7 @@ __device__ void fire_block(const KArgs& a, const PopBufs& pb, uint32_t b, const 
 	do {
 		for (int k = G.rank; k < NG; k += TPP) cgen[k] = gen[k] + dt * vel[k];
 		G.sync();
-		const float ce = score_pose<TPP, true>(a.L, cgen, cgrad, S.pose, G);
+		const float ce = score_pose<TPP, true, false, false, SUMS>(a.L, cgen, cgrad, S.pose, G);
 		float pw = 0.f;
 		for (int k = G.rank; k < NG; k += TPP) pw += -cgrad[k] * vel[k];
 		const float power = G.sum(pw);
@@ -288,7 +295,7 @@ __device__ void fire_block(const KArgs& a, const PopBufs& pb, uint32_t b, const 
 // ---------------------------------------------------------------------------
 // Solis-Wets with SWAT3 step scaling (cuda/kernel3.cu:30-308).
 // ---------------------------------------------------------------------------
-template <int TPP>
+template <int TPP, int SUMS = TPP>
 __device__ void sw_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
 {
 	const int P = a.dp.pop_size, NG = a.dp.num_of_genes;
@@ -324,7 +331,7 @@ __device__ void sw_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Gr
 		G.sync();
 		for (int k = gs + G.rank; k < NG; k += TPP) cand[k] = gen[k] + dev[k] + bias[k];
 		G.sync();
-		float ce = score_pose<TPP, false>(a.L, cand, nullptr, S.pose, G);
+		float ce = score_pose<TPP, false, false, false, SUMS>(a.L, cand, nullptr, S.pose, G);
 		evals++;
 		if (ce < cur_e) {
 			for (int k = gs + G.rank; k < NG; k += TPP) { gen[k] = cand[k]; bias[k] = 0.6f * bias[k] + 0.4f * dev[k]; }
@@ -332,7 +339,7 @@ __device__ void sw_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Gr
 		} else {
 			for (int k = gs + G.rank; k < NG; k += TPP) cand[k] = gen[k] - dev[k] - bias[k];
 			G.sync();
-			ce = score_pose<TPP, false>(a.L, cand, nullptr, S.pose, G);
+			ce = score_pose<TPP, false, false, false, SUMS>(a.L, cand, nullptr, S.pose, G);
 			evals++;
 			if (ce < cur_e) {
 				for (int k = gs + G.rank; k < NG; k += TPP) { gen[k] = cand[k]; bias[k] = 0.6f * bias[k] - 0.4f * dev[k]; }
@@ -377,7 +384,7 @@ __device__ __forceinline__ void warp_minimum2(int lane, float& v, int& k)
 	}
 }
 
-template <int TPP>
+template <int TPP, int SUMS = TPP>
 __device__ void ga_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
 {
 	const int P = a.dp.pop_size, NG = a.dp.num_of_genes;
@@ -459,51 +466,51 @@ __device__ void ga_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Gr
 		a.prng[b * T + r] = s;
 	}
 	G.sync();
-	const float e = score_pose<TPP, false>(a.L, off, nullptr, S.pose, G);
+	const float e = score_pose<TPP, false, false, false, SUMS>(a.L, off, nullptr, S.pose, G);
 	if (G.rank == 0) { pb.e[b] = e; a.evals_new[b] = 1; }
 	for (int g = G.rank; g < NG; g += TPP) pb.conf[(size_t)b * kGenotypeStride + g] = off[g];
 	G.sync();
 }
 
 // The blocks above on the launch's own population buffers.
-template <int TPP, int METHOD>
+template <int TPP, int METHOD, int SUMS = TPP>
 __device__ __forceinline__ void gradient_ls_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
-{ gradient_ls_block<TPP, METHOD>(a, bufs_of(a), b, G, S); }
-template <int TPP>
+{ gradient_ls_block<TPP, METHOD, SUMS>(a, bufs_of(a), b, G, S); }
+template <int TPP, int SUMS = TPP>
 __device__ __forceinline__ void fire_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
-{ fire_block<TPP>(a, bufs_of(a), b, G, S); }
-template <int TPP>
+{ fire_block<TPP, SUMS>(a, bufs_of(a), b, G, S); }
+template <int TPP, int SUMS = TPP>
 __device__ __forceinline__ void sw_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
-{ sw_block<TPP>(a, bufs_of(a), b, G, S); }
-template <int TPP>
+{ sw_block<TPP, SUMS>(a, bufs_of(a), b, G, S); }
+template <int TPP, int SUMS = TPP>
 __device__ __forceinline__ void ga_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
-{ ga_block<TPP>(a, bufs_of(a), b, G, S); }
+{ ga_block<TPP, SUMS>(a, bufs_of(a), b, G, S); }
 
 // Initial population energies (cuda/kernel1.cu:26-55).
-template <int TPP>
+template <int TPP, int SUMS = TPP>
 __device__ void initpop_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
 {
 	const int NG = a.dp.num_of_genes;
 	for (int k = G.rank; k < NG; k += TPP) S.gen[k] = pb.conf[(size_t)b * kGenotypeStride + k];
 	G.sync();
-	const float e = score_pose<TPP, false>(a.L, S.gen, nullptr, S.pose, G);
+	const float e = score_pose<TPP, false, false, false, SUMS>(a.L, S.gen, nullptr, S.pose, G);
 	if (G.rank == 0) { pb.e[b] = e; a.evals_new[b] = 1; }
 	G.sync();
 }
 
-template <int TPP>
+template <int TPP, int SUMS = TPP>
 __device__ __forceinline__ void initpop_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
-{ initpop_block<TPP>(a, bufs_of(a), b, G, S); }
+{ initpop_block<TPP, SUMS>(a, bufs_of(a), b, G, S); }
 
 // Stand-alone scorer: energies (and gradients when a.conf_cur != nullptr is
 // used as the gradient output) of nblocks genotypes.
-template <int TPP, bool GRAD>
+template <int TPP, bool GRAD, int SUMS = TPP>
 __device__ void score_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S, float* grads)
 {
 	const int NG = a.dp.num_of_genes;
 	for (int k = G.rank; k < NG; k += TPP) S.gen[k] = a.conf[(size_t)b * kGenotypeStride + k];
 	G.sync();
-	const float e = score_pose<TPP, GRAD>(a.L, S.gen, S.grad, S.pose, G);
+	const float e = score_pose<TPP, GRAD, false, false, SUMS>(a.L, S.gen, S.grad, S.pose, G);
 	if (GRAD)
 		for (int k = G.rank; k < NG; k += TPP) grads[(size_t)b * kGenotypeStride + k] = S.grad[k];
 	if (G.rank == 0) a.e[b] = e;

@@ -210,11 +210,11 @@ __device__ int pipe_take(const PipeArgs& p, int worker, const Group<TPP>& G, int
 }
 
 // The GA step of a task; GA_TPP < TPP: by the group's first warp.
-template <int TPP, int GA_TPP>
+template <int TPP, int GA_TPP, int SUMS>
 __device__ __forceinline__ void pipe_ga(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
 {
 	if constexpr (GA_TPP == TPP) {
-		ga_block<TPP>(a, pb, b, G, S);
+		ga_block<TPP, SUMS>(a, pb, b, G, S);
 	} else {
 		static_assert(GA_TPP == 32, "the GA step takes the whole group or its first warp");
 		if (G.rank < 32) {
@@ -230,7 +230,7 @@ __device__ __forceinline__ void pipe_ga(const KArgs& a, const PopBufs& pb, uint3
 
 // AS: a docking with AutoStop (its own instantiation: the test's code in the
 // kernel of a docking without it cost that one 4 %).
-template <int TPP, int LSMET, int GA_TPP, bool AS>
+template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS>
 __device__ void pipe_worker(const PipeArgs& p)
 {
 	extern __shared__ __align__(16) char smem[];
@@ -238,7 +238,7 @@ __device__ void pipe_worker(const PipeArgs& p)
 	char* base = smem + (size_t)local * p.group_bytes;
 	PipeHdr& H = *reinterpret_cast<PipeHdr*>(base);
 	const LigDev& L0 = p.ka.L;
-	const GroupSmem S = carve_group(base + kPipeHdrBytes, L0.natoms, L0.ntors, 64, TPP);
+	const GroupSmem S = carve_group(base + kPipeHdrBytes, L0.natoms, L0.ntors, 64, TPP, ep_records(L0, TPP, SUMS));
 	Group<TPP> G;
 	G.rank = threadIdx.x % TPP;
 	G.bar_id = 1 + local;
@@ -271,12 +271,12 @@ __device__ void pipe_worker(const PipeArgs& p)
 			const KArgs& a = p.ka;
 			const PopBufs pb = p.bufs[g & (p.nbuf - 1)];
 			const uint32_t b = (uint32_t)(run * P + ent);
-			pipe_ga<TPP, GA_TPP>(a, pb, b, G, S);
+			pipe_ga<TPP, GA_TPP, SUMS>(a, pb, b, G, S);
 			// num_of_lsentities == pop_size: local-search block b is entity b
-			if constexpr (LSMET == LS_SW) sw_block<TPP>(a, pb, b, G, S);
-			else if constexpr (LSMET == LS_AD) gradient_ls_block<TPP, LS_AD>(a, pb, b, G, S);
-			else if constexpr (LSMET == LS_ADAM) gradient_ls_block<TPP, LS_ADAM>(a, pb, b, G, S);
-			else fire_block<TPP>(a, pb, b, G, S);
+			if constexpr (LSMET == LS_SW) sw_block<TPP, SUMS>(a, pb, b, G, S);
+			else if constexpr (LSMET == LS_AD) gradient_ls_block<TPP, LS_AD, SUMS>(a, pb, b, G, S);
+			else if constexpr (LSMET == LS_ADAM) gradient_ls_block<TPP, LS_ADAM, SUMS>(a, pb, b, G, S);
+			else fire_block<TPP, SUMS>(a, pb, b, G, S);
 		}
 		__threadfence();
 		G.sync();
@@ -392,10 +392,10 @@ __device__ void pipe_worker(const PipeArgs& p)
 
 constexpr int pipe_min_ctas(int lsmet) { return lsmet == LS_SW ? ADGPU_PIPE_MIN_CTAS_SW : ADGPU_PIPE_MIN_CTAS; }
 
-template <int TPP, int LSMET, int GA_TPP, bool AS>
+template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS>
 __global__ void __launch_bounds__(kPipeThreads, pipe_min_ctas(LSMET)) pipe_kernel(const PipeArgs p)
 {
-	pipe_worker<TPP, LSMET, GA_TPP, AS>(p);
+	pipe_worker<TPP, LSMET, GA_TPP, AS, SUMS>(p);
 }
 
 // Check 0 (before the first generation) and the first generation's GA tasks.
@@ -465,10 +465,10 @@ __global__ void __launch_bounds__(256) pipe_final_kernel(PipeArgs p, long long* 
 // Initial check and tasks, the persistent launch, the final accounting; the
 // grid is sized from the kernel's occupancy (persistent: every pose group a
 // worker) and capped by the entities a generation offers.
-template <int TPP, int LSMET, int GA_TPP, bool AS>
+template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS>
 static adgpu_status launch_pipe_as(PipeArgs p, long long* d_out, cudaStream_t st)
 {
-	auto kfn = pipe_kernel<TPP, LSMET, GA_TPP, AS>;
+	auto kfn = pipe_kernel<TPP, LSMET, GA_TPP, AS, SUMS>;
 	const int gpc = kPipeThreads / TPP;
 	const int bytes = p.group_bytes * gpc;
 	if (bytes > 48 * 1024) ADGPU_CUDA_RET(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "pipeline smem");
@@ -491,11 +491,11 @@ static adgpu_status launch_pipe_as(PipeArgs p, long long* d_out, cudaStream_t st
 	return ADGPU_OK;
 }
 
-template <int TPP, int LSMET, int GA_TPP = TPP>
+template <int TPP, int LSMET, int GA_TPP = TPP, int SUMS = TPP>
 static adgpu_status launch_pipe(const PipeArgs& p, long long* d_out, cudaStream_t st)
 {
-	if (p.as_state) return launch_pipe_as<TPP, LSMET, GA_TPP, true>(p, d_out, st);
-	if constexpr (GA_TPP == TPP) return launch_pipe_as<TPP, LSMET, GA_TPP, false>(p, d_out, st);
+	if (p.as_state) return launch_pipe_as<TPP, LSMET, GA_TPP, true, SUMS>(p, d_out, st);
+	if constexpr (GA_TPP == TPP && SUMS == TPP) return launch_pipe_as<TPP, LSMET, GA_TPP, false, SUMS>(p, d_out, st);
 	else return fail(ADGPU_ERR_ARG, "GA group size");
 }
 
@@ -549,6 +549,9 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 	if (tpp != 32 && tpp != 64 && tpp != 128) return fail(ADGPU_ERR_ARG, "threads per pose must be 32, 64 or 128");
 	const int ga_tpp = as.frequency ? as.ga_tpp : tpp;
 	if (ga_tpp != tpp && (ga_tpp != 32 || tpp != 64)) return fail(ADGPU_ERR_ARG, "GA group size");
+	// 128 threads with the sums of 64: a docking that leaves SMs short of work
+	const bool share = as.share && tpp == 64;
+	if (share) tpp = 128;
 	const int P = dp.pop_size;
 	const size_t n = (size_t)runs * P;
 	const int nbuf = pipeline_buffers(tpp);
@@ -599,7 +602,7 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 	long long* d_out = reinterpret_cast<long long*>(m + o_ctl + al(sizeof(PipeCtl)));
 	p.runs = (int)runs; p.pop = P;
 	p.max_evals = max_evals; p.max_gens = max_gens;
-	p.group_bytes = kPipeHdrBytes + group_smem_bytes(base.L.natoms, base.L.ntors, 64, tpp);
+	p.group_bytes = kPipeHdrBytes + group_smem_bytes(base.L.natoms, base.L.ntors, 64, tpp, ep_records(base.L, tpp, share ? 64 : tpp));
 
 	cudaStream_t st = 0;   // the legacy stream: ordered after the caller's initial-population calls
 	// the library's population buffers start as zeros, like the caller's
@@ -635,7 +638,16 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 		else if (ga_tpp == 32) rc = fail(ADGPU_ERR_ARG, "GA group size");
 		else ADGPU_PIPE_LSMET(64)
 		break;
-	default: ADGPU_PIPE_LSMET(128) break;
+	default:
+		if (!share) ADGPU_PIPE_LSMET(128)
+		else if (ga_tpp == 32 && lsmet == 0) rc = launch_pipe<128, LS_SW, 32, 64>(p, d_out, st);
+		else if (ga_tpp == 32 && lsmet == 1) rc = launch_pipe<128, LS_AD, 32, 64>(p, d_out, st);
+		else if (ga_tpp == 32) rc = fail(ADGPU_ERR_ARG, "GA group size");
+		else if (lsmet == 0) rc = launch_pipe<128, LS_SW, 128, 64>(p, d_out, st);
+		else if (lsmet == 1) rc = launch_pipe<128, LS_AD, 128, 64>(p, d_out, st);
+		else if (lsmet == 2) rc = launch_pipe<128, LS_ADAM, 128, 64>(p, d_out, st);
+		else rc = launch_pipe<128, LS_FIRE, 128, 64>(p, d_out, st);
+		break;
 	}
 #undef ADGPU_PIPE_LSMET
 	if (rc != ADGPU_OK) return rc;

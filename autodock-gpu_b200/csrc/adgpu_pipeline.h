@@ -28,6 +28,7 @@ struct PipeAutoStop {
 	uint32_t frequency = 0;          // generations between checks
 	float stopstd = 0.0f;
 	unsigned long long min_evals = 0;
+	bool share = false;              // 128 threads per pose with the sums of 64 (shares_sums)
 	int ga_tpp = 0;                  // threads per pose of the GA step (the searches' own, or 32 where they take 64)
 };
 
@@ -36,6 +37,9 @@ struct PipeAutoStop {
 // which holds when the local-search rate is 100 % (num_of_lsentities ==
 // pop_size, host/src/performdocking.cpp.Cuda:446).
 bool pipeline_applies(const adgpu_dockpars& dp, uint32_t runs);
+
+// Threads per pose of a pipelined docking when none is configured.
+int pipeline_default_tpp(int lsmet, long tasks);
 
 // The generation loop of docking_with_gpu as one persistent launch; the
 // arguments and results are those of adgpu_dock_resident_autostop.  tpp 0: default.
