@@ -226,7 +226,9 @@ static int auto_tpp(uint32_t n, int kind)
 	return (long)n * 2 <= groups32 ? 64 : 32;
 }
 
-// Pose groups of 128 threads per SM up to which they beat twice as many of 64.
+// Pose groups of 128 threads per SM up to which they beat twice as many of 64
+// (33-atom-ligand host loop, ADADELTA, 8 generations, B200: one run 8.5 -> 7.2
+// ms, three 10.0 -> 8.4; at five a group more runs as many rounds as 64's).
 constexpr long kShareGroupsPerSm = 4;
 
 template <int KIND>
@@ -234,9 +236,9 @@ adgpu_status launch_kind(const KArgs& a, float* grads, cudaStream_t stream, int 
 {
 	if (tpp == 0) {
 		tpp = auto_tpp(a.nblocks, KIND);
-		// a launch that leaves SMs short of work takes 128 threads per pose
-		// with the sums of 64, so its results stay those of 64
-		if constexpr (KIND != 8)
+		// a launch with gradients that leaves SMs short of work takes 128
+		// threads per pose with the sums of 64: its results stay those of 64
+		if constexpr ((KIND >= 2 && KIND <= 4) || KIND == 7)
 			if (tpp == 64 && shares_sums(a.L) && (long)a.nblocks <= kShareGroupsPerSm * (long)g_num_sms)
 				return launch_lga<128, KIND, 64>(a, grads, stream, 128);
 	}
@@ -303,7 +305,18 @@ adgpu_status dock_resident(ApiState& s, int lsmet, uint32_t runs, uint64_t max_e
 	// (an AutoStop test sums all energies in one thread: with many of them it
 	// would outlast the pipelined loop's idle limit)
 	const bool as_fits = as_frequency == 0 || (uint64_t)runs * (uint64_t)dp.pop_size <= (1u << 18);
-	if (s.pipeline && as_fits && pipeline_applies(dp, runs)) {
+	if (g_num_sms == 0) {
+		int dev; ADGPU_CUDA(cudaGetDevice(&dev), "device");
+		ADGPU_CUDA(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev), "sm count");
+	}
+	const long tasks = (long)runs * dp.pop_size;
+	// ADAM and FIRE run a fixed number of iterations: entities that all run at
+	// once end together, so with AutoStop there is nothing to work ahead of.
+	// (36-atom ligand, 39 runs, B200, pipelined against synchronous: ADAM 35.9
+	// and 41.4 ms, FIRE 44.4 and 43.3; 5 runs 9.8 and 9.4, 12.8 and 10.9.)
+	const bool as_gains = as_frequency == 0 || lsmet < 2 ||
+	                      (lsmet == 2 && tasks > 4L * ADGPU_MIN_CTAS_GRAD * g_num_sms);
+	if (s.pipeline && as_fits && as_gains && pipeline_applies(dp, runs)) {
 		*autostopped = 0;
 		KArgs base = make_args(s);
 		PipeAutoStop as;
@@ -317,7 +330,12 @@ adgpu_status dock_resident(ApiState& s, int lsmet, uint32_t runs, uint64_t max_e
 			as.ga_tpp = tpp ? tpp : auto_tpp(runs * (uint32_t)dp.pop_size, 0);
 			if (tpp == 0) {
 				tpp = auto_tpp(runs * dp.num_of_lsentities, lsmet + 1);
-				as.share = tpp == 64 && shares_sums(base.L) && pipeline_default_tpp(lsmet, (long)runs * dp.pop_size) == 128;
+				// 128 threads with the sums of 64, up to five entities a group,
+				// with ADADELTA (36-atom ligand, B200, against 64 threads: 20
+				// runs 30.0 and 33.8 ms, 25 runs 35.1 and 36.5, 30 runs 41.4 and
+				// 39.0).  Solis-Wets' scoring has no gradient to share out (12
+				// runs 13.5 and 12.7 ms).
+				as.share = tpp == 64 && lsmet == 1 && shares_sums(base.L) && tasks <= 5L * ADGPU_MIN_CTAS_GRAD * g_num_sms;
 			}
 		}
 		return dock_pipelined(base, s.pipe, lsmet, tpp, runs, max_evals, max_gens, as, c1, e1, c2, e2,

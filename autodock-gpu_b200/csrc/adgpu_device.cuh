@@ -719,7 +719,9 @@ __host__ __device__ inline bool shares_sums(const LigDev& L)
 // are loaded ahead of the sines and cosines, and with up to 64 atoms the upper
 // two warps take the intermolecular terms while the lower two, which built
 // the pose, start on the pairs (a docking of one run 24.4 -> 21.0 ms; the
-// early loads lost 2 % at 64 threads and 32).  Every float is computed by the same operations in the same
+// early loads lost 2 % at 64 threads and 32; without gradients the extra
+// barrier cost more than the terms, a Solis-Wets docking of three runs 10.7 ->
+// 11.4 ms).  Every float is computed by the same operations in the same
 // order whatever the group does in parallel, and each thread adds up the same
 // terms: results do not depend on it.
 //
@@ -735,7 +737,7 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 	// the upper half takes the lower half's intermolecular terms
 	constexpr bool kCanSplit = TPP == 128 && !TERMS && !REF_GRID;
 	static_assert(SUMS == TPP || (SUMS == 64 && kCanSplit), "sums of another group size");
-	const bool split = kCanSplit && (SUMS != TPP || L.natoms <= TPP / 2);
+	const bool split = kCanSplit && (SUMS != TPP || (GRAD && L.natoms <= TPP / 2));
 
 	// 0. this thread's first atom (with split, the upper half's: its partner's)
 	struct AtomIn { float4 r; uint32_t info, chain; int len; };

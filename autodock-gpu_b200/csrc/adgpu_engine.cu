@@ -331,10 +331,10 @@ __device__ void engine_worker(const TickArgs& t, const TickClass& C)
 		const int c = rq.cur[run];
 		if (phase == 0) {
 			// step 0: the initial population's energies (cuda/kernel1.cu:26-55)
-			initpop_block<TPP>(a, PopBufs{nullptr, nullptr, rq.conf[c], rq.e[c]}, (uint32_t)(run * P + idx), G, S);
+			initpop_block<TPP>(a, PopBufs{nullptr, nullptr, rq.conf[c], rq.e[c], 0}, (uint32_t)(run * P + idx), G, S);
 		} else {
 			const bool ls_phase = (phase & 1u) != 0;
-			if (!ls_phase) ga_block<TPP>(a, PopBufs{rq.conf[c], rq.e[c], rq.conf[c ^ 1], rq.e[c ^ 1]},
+			if (!ls_phase) ga_block<TPP>(a, PopBufs{rq.conf[c], rq.e[c], rq.conf[c ^ 1], rq.e[c ^ 1], 0},
 			                             (uint32_t)(run * P + idx), G, S);
 			if (ls_phase || (fused && L > 0)) {
 				// local-search block run*L + idx; entity l of run r draws from
@@ -344,7 +344,7 @@ __device__ void engine_worker(const TickArgs& t, const TickClass& C)
 					if (G.rank == 0) a.prng = rq.a.prng + (size_t)run * (size_t)(P - L) * 64;
 					G.sync();
 				}
-				const PopBufs pb{nullptr, nullptr, rq.conf[c ^ 1], rq.e[c ^ 1]};
+				const PopBufs pb{nullptr, nullptr, rq.conf[c ^ 1], rq.e[c ^ 1], 0};
 				const uint32_t b = (uint32_t)(run * L + idx);
 				if constexpr (LSMET == LS_SW) sw_block<TPP>(a, pb, b, G, S);
 				else if constexpr (LSMET == LS_AD) gradient_ls_block<TPP, LS_AD>(a, pb, b, G, S);

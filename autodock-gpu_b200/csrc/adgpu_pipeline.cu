@@ -269,14 +269,15 @@ __device__ void pipe_worker(const PipeArgs& p)
 		// only count down
 		if (!H.stopped) {
 			const KArgs& a = p.ka;
-			const PopBufs pb = p.bufs[g & (p.nbuf - 1)];
+			PopBufs pb = p.bufs[g & (p.nbuf - 1)];
+			pb.gen = g;
 			const uint32_t b = (uint32_t)(run * P + ent);
 			pipe_ga<TPP, GA_TPP, SUMS>(a, pb, b, G, S);
 			// num_of_lsentities == pop_size: local-search block b is entity b
-			if constexpr (LSMET == LS_SW) sw_block<TPP, SUMS>(a, pb, b, G, S);
-			else if constexpr (LSMET == LS_AD) gradient_ls_block<TPP, LS_AD, SUMS>(a, pb, b, G, S);
-			else if constexpr (LSMET == LS_ADAM) gradient_ls_block<TPP, LS_ADAM, SUMS>(a, pb, b, G, S);
-			else fire_block<TPP, SUMS>(a, pb, b, G, S);
+			if constexpr (LSMET == LS_SW) sw_block<TPP, SUMS, true>(a, pb, b, G, S);
+			else if constexpr (LSMET == LS_AD) gradient_ls_block<TPP, LS_AD, SUMS, true>(a, pb, b, G, S);
+			else if constexpr (LSMET == LS_ADAM) gradient_ls_block<TPP, LS_ADAM, SUMS, true>(a, pb, b, G, S);
+			else fire_block<TPP, SUMS, true>(a, pb, b, G, S);
 		}
 		__threadfence();
 		G.sync();
@@ -592,7 +593,7 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 	p.ka.conf = p.ka.e = nullptr;
 	p.nbuf = nbuf;
 	for (int k = 0; k < nbuf; k++)
-		p.bufs[k] = PopBufs{conf[k], en[k], conf[(k + 1) % nbuf], en[(k + 1) % nbuf]};
+		p.bufs[k] = PopBufs{conf[k], en[k], conf[(k + 1) % nbuf], en[(k + 1) % nbuf], 0};
 	p.next = reinterpret_cast<unsigned long long*>(m + o_slots);
 	p.idle_ns = 2000000000ll;
 	int* ri = reinterpret_cast<int*>(m + o_runs);
@@ -600,6 +601,7 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 	p.started = ri; p.done = ri + rs; p.comp = ri + 2 * rs; p.pending = ri + 3 * rs; p.inc = ri + 4 * rs;
 	p.ctl = reinterpret_cast<PipeCtl*>(m + o_ctl);
 	long long* d_out = reinterpret_cast<long long*>(m + o_ctl + al(sizeof(PipeCtl)));
+	p.ka.abandon = &p.ctl->stop_gen;
 	p.runs = (int)runs; p.pop = P;
 	p.max_evals = max_evals; p.max_gens = max_gens;
 	p.group_bytes = kPipeHdrBytes + group_smem_bytes(base.L.natoms, base.L.ntors, 64, tpp, ep_records(base.L, tpp, share ? 64 : tpp));
@@ -640,13 +642,9 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 		break;
 	default:
 		if (!share) ADGPU_PIPE_LSMET(128)
-		else if (ga_tpp == 32 && lsmet == 0) rc = launch_pipe<128, LS_SW, 32, 64>(p, d_out, st);
-		else if (ga_tpp == 32 && lsmet == 1) rc = launch_pipe<128, LS_AD, 32, 64>(p, d_out, st);
-		else if (ga_tpp == 32) rc = fail(ADGPU_ERR_ARG, "GA group size");
-		else if (lsmet == 0) rc = launch_pipe<128, LS_SW, 128, 64>(p, d_out, st);
-		else if (lsmet == 1) rc = launch_pipe<128, LS_AD, 128, 64>(p, d_out, st);
-		else if (lsmet == 2) rc = launch_pipe<128, LS_ADAM, 128, 64>(p, d_out, st);
-		else rc = launch_pipe<128, LS_FIRE, 128, 64>(p, d_out, st);
+		else if (lsmet != 1) rc = fail(ADGPU_ERR_ARG, "shared sums");
+		else if (ga_tpp == 32) rc = launch_pipe<128, LS_AD, 32, 64>(p, d_out, st);
+		else rc = launch_pipe<128, LS_AD, 128, 64>(p, d_out, st);
 		break;
 	}
 #undef ADGPU_PIPE_LSMET
