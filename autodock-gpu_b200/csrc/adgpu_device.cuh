@@ -506,8 +506,9 @@ __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, i
 	const uint32_t* pw = reinterpret_cast<const uint32_t*>(L.pairs2 + (rank / 32) * kBlock + 96) + (rank % 32);
 	// Groups of 128 load a step's record during the step before: they score
 	// few poses per SM, so a step's latency counts, and they have the registers.
-	// (With 64 threads it lost 2 to 4 %.)
-	constexpr bool kAhead = TPP == 128;
+	// (With 64 threads it lost 2 to 4 %; without gradients the Solis-Wets
+	// kernels' 72 registers do not hold it.)
+	constexpr bool kAhead = TPP == 128 && GRAD;
 	uint32_t wa = 0, wb = 0;
 	float4 q0, q1, q2;
 	q0 = q1 = q2 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -752,7 +753,7 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 		}
 		return x;
 	};
-	constexpr bool kEarly = TPP == 128;
+	constexpr bool kEarly = TPP == 128 && (GRAD || SUMS != TPP);
 	const int a0 = split ? rank & (TPP / 2 - 1) : rank;
 	AtomIn in;
 	in.r = make_float4(0.f, 0.f, 0.f, 0.f);
