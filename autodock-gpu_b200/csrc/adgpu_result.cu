@@ -95,14 +95,17 @@ __device__ int plain_rank(const T* e, int n, int i)
 	return rank;
 }
 
+// V: float4, or float for populations that are not 16-byte aligned.
+template <class V>
 __global__ void __launch_bounds__(256) arrange_kernel(float* pop, float* energies, float* scratch, int P)
 {
+	constexpr int kPer = 64 * (int)sizeof(float) / (int)sizeof(V);      // of a genotype
 	extern __shared__ float sh_e[];
 	int* dst = reinterpret_cast<int*>(sh_e + P);
 	const size_t r = blockIdx.x;
 	float* E = energies + r * P;
-	float4* G = reinterpret_cast<float4*>(pop + r * P * 64);
-	float4* S = reinterpret_cast<float4*>(scratch + r * P * 64);
+	V* G = reinterpret_cast<V*>(pop + r * P * 64);
+	V* S = reinterpret_cast<V*>(scratch + r * P * 64);
 	int nans = 0;
 	for (int i = threadIdx.x; i < P; i += blockDim.x) {
 		const float e = E[i];
@@ -112,10 +115,10 @@ __global__ void __launch_bounds__(256) arrange_kernel(float* pop, float* energie
 	nans = __syncthreads_or(nans);
 	for (int i = threadIdx.x; i < P; i += blockDim.x) dst[i] = nans ? stable_rank(sh_e, P, i) : plain_rank(sh_e, P, i);
 	__syncthreads();
-	for (int k = threadIdx.x; k < P * 16; k += blockDim.x) S[dst[k >> 4] * 16 + (k & 15)] = G[k];
+	for (int k = threadIdx.x; k < P * kPer; k += blockDim.x) S[dst[k / kPer] * kPer + k % kPer] = G[k];
 	for (int i = threadIdx.x; i < P; i += blockDim.x) E[dst[i]] = sh_e[i];
 	__syncthreads();
-	for (int k = threadIdx.x; k < P * 16; k += blockDim.x) G[k] = S[k];
+	for (int k = threadIdx.x; k < P * kPer; k += blockDim.x) G[k] = S[k];
 }
 
 // ---------------------------------------------------------------------------
@@ -823,7 +826,10 @@ adgpu_status process_result_core(const PostLigand& L, const uint32_t* pairs, con
 	adgpu_cluster* d_cl = (adgpu_cluster*)(d + o_cl);
 	int* d_nc = (int*)(d + o_nc);
 
-	arrange_kernel<<<R, 256, (size_t)P * 8, st>>>(populations, energies, (float*)(d + o_scr), P);
+	if (reinterpret_cast<uintptr_t>(populations) % sizeof(float4) == 0)
+		arrange_kernel<float4><<<R, 256, (size_t)P * 8, st>>>(populations, energies, (float*)(d + o_scr), P);
+	else
+		arrange_kernel<float><<<R, 256, (size_t)P * 8, st>>>(populations, energies, (float*)(d + o_scr), P);
 	const int ntask = params->rescore_entities ? R * P : R;
 	const size_t wsm = (size_t)kWarps * rescore_warp_bytes(N, NR);
 	if (wsm > 48 * 1024) {

@@ -108,3 +108,20 @@ def test_rescored_energies(flex):
     assert (np.abs(got - want) <= 0.06 * size + 0.02)[inside].all()
     best = np.array([[r.inter_e, r.interflex_e, r.intra_e, r.intraflex_e] for r in out.runs])
     np.testing.assert_allclose(best.sum(1), out.entities[:, 0, :2].sum(1), rtol=1e-6)
+
+
+def test_populations_aligned_to_a_float():
+    """Populations anywhere a float may lie: ordered as 16-byte aligned ones."""
+    runs, pop = 3, 7
+    grid, lig, pops, en = inputs(runs, pop)
+    layout = torch.from_numpy(grid.reference_layout()).cuda()
+    for off in (0, 1, 2):
+        dev = torch.zeros(pops.size + off, device="cuda")[off:].view(pops.shape)
+        assert dev.data_ptr() % 16 == 4 * off
+        dev.copy_(torch.from_numpy(pops))
+        de = torch.zeros(en.size + off, device="cuda")[off:]
+        de.copy_(torch.from_numpy(en))
+        result.process_result(lig, layout, dev, de, runs)
+        perm = np.concatenate([r * pop + stable_order(en[r * pop:(r + 1) * pop]) for r in range(runs)])
+        np.testing.assert_array_equal(dev.cpu().numpy(), pops[perm])
+        np.testing.assert_array_equal(de.cpu().numpy(), en[perm])
