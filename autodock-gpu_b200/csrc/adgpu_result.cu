@@ -695,6 +695,16 @@ size_t put(std::vector<unsigned char>& blob, const T* src, size_t n)
 	return off;
 }
 
+// Raises a kernel's dynamic shared-memory limit.  The limit belongs to the
+// function, not to a launch, so bytes is the most that any call asks for: a
+// call's own size would lower the limit of one that another thread is about to
+// launch.
+template <class F>
+cudaError_t allow_smem(F* kernel, size_t bytes)
+{
+	return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 }  // namespace
 }  // namespace adgpu
 
@@ -833,7 +843,7 @@ adgpu_status process_result_core(const PostLigand& L, const uint32_t* pairs, con
 	const int ntask = params->rescore_entities ? R * P : R;
 	const size_t wsm = (size_t)kWarps * rescore_warp_bytes(N, NR);
 	if (wsm > 48 * 1024) {
-		e = cudaFuncSetAttribute(rescore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
+		e = allow_smem(rescore_kernel, (size_t)kWarps * rescore_warp_bytes(ADGPU_MAX_ATOMS, ADGPU_MAX_ROTBONDS));
 		if (e != cudaSuccess) return done(e, "result smem");
 	}
 	int dev = 0, sms = 148;
@@ -856,14 +866,13 @@ adgpu_status process_result_core(const PostLigand& L, const uint32_t* pairs, con
 			pair_rmsd_kernel<<<std::min((npair + kWarps - 1) / kWarps, sms * 16), kWarps * 32, (size_t)kWarps * N * 8, st>>>(
 			    D, R, d_bx, d_ord, tol, mat, bits);
 		const size_t rows = (size_t)R * W * 4;
-		if (e == cudaSuccess && rows > 40 * 1024)
-			e = cudaFuncSetAttribute(cluster_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows);
+		if (e == cudaSuccess && rows > 40 * 1024) e = allow_smem(cluster_scan_kernel, (size_t)kPairRuns * kPairRuns / 8);
 		if (e == cudaSuccess)
 			cluster_scan_kernel<<<1, 256, rows, st>>>(R, d_runs, d_ord, mat, bits, params->nr_cluster_poses, free_roaming,
 			                                          torsional, d_cl, d_nc);
 	} else {
 		const size_t csm = (size_t)32 * N * 8;
-		if (csm > 48 * 1024) e = cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
+		if (csm > 48 * 1024) e = allow_smem(cluster_kernel, (size_t)32 * ADGPU_MAX_ATOMS * 8);
 		if (e == cudaSuccess)
 			cluster_kernel<<<1, 1024, csm, st>>>(D, R, d_runs, d_bx, d_ord, (int*)(d + o_cen), (double*)(d + o_cr), tol,
 			                                     params->nr_cluster_poses, free_roaming, torsional, d_cl, d_nc);

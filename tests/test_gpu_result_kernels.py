@@ -6,6 +6,8 @@ that does not, and re-scored energies with and without flexible residues.
 The RMSDs and clusters are checked against a plain restatement of
 generate_output's greedy clustering (host/src/processresult.cpp:688-746) on
 the returned poses."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -125,3 +127,33 @@ def test_populations_aligned_to_a_float():
         perm = np.concatenate([r * pop + stable_order(en[r * pop:(r + 1) * pop]) for r in range(runs)])
         np.testing.assert_array_equal(dev.cpu().numpy(), pops[perm])
         np.testing.assert_array_equal(de.cpu().numpy(), en[perm])
+
+
+def test_calls_of_several_threads():
+    """Calls of different run counts at the same time: the clustering's shared
+    memory grows with the runs (66 KB at 720, 128 KB at 1,024)."""
+    pop, sizes, errors, labels = 2, (720, 1024), [], {}
+    jobs = {}
+    for runs in sizes:
+        grid, lig, pops, en = inputs(runs, pop)
+        jobs[runs] = (lig, torch.from_numpy(grid.reference_layout()).cuda(), torch.from_numpy(pops).cuda(), torch.from_numpy(en).cuda())
+        out = result.process_result(*jobs[runs], runs)
+        labels[runs] = [r.cluster_id for r in out.runs]
+    start = threading.Barrier(4)
+
+    def worker(runs):
+        lig, layout, pops, en = jobs[runs][0], *[t.clone() for t in jobs[runs][1:]]
+        torch.cuda.synchronize()
+        start.wait()
+        try:
+            for _ in range(25):
+                assert [r.cluster_id for r in result.process_result(lig, layout, pops, en, runs).runs] == labels[runs]
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=worker, args=(r,)) for r in sizes * 2]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
