@@ -414,6 +414,14 @@ __device__ __forceinline__ float lt1(float a, float b)
 	return r;
 }
 
+// The larger of a and b; NaN where either is.
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+	float r;
+	asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	return r;
+}
+
 // inv^e by squaring (the general-exponent path of modified pair potentials)
 static __device__ __noinline__ float pow_int(float b, int e)
 {
@@ -446,17 +454,25 @@ __device__ __forceinline__ void pair_force(int* f3, uint32_t i, uint32_t j, floa
 // wrap, and every atom's forces start at minus the sum of its offsets over
 // the ligand's records (L.f3_bias, from the tables), so they end exact.
 __device__ __forceinline__ float clamp_term(float v) { return fminf(kMaxTerm, fmaxf(-kMaxTerm, v)); }
-// pg: the pairs' forces along their axes, unscaled.  A component is at most
-// that times 1024 (and rounding), so a warp whose pairs are all below 7.999 in
-// size needs no clamp: most steps of a search, 12 instructions each (docking
-// of 100 runs, ADADELTA, B200: 126.6 -> 125.6 ms).  NaN and infinity fail the
-// test.
-__device__ __forceinline__ void couple_force(unsigned* f3, uint32_t c, uint32_t i, uint32_t j, float2 gx, float2 gy, float2 gz,
-                                             float2 pg)
+// g = s * gdd: the pairs' forces, s their axes.  pg: the forces' sizes,
+// unscaled, NaN where the distance r is NaN.  A component is at most pg times
+// 1024 (and rounding), so a warp whose pairs are all below 7.999 in size needs
+// no clamp: most steps of a search, 12 instructions each (docking of 100 runs,
+// ADADELTA, B200: 126.6 -> 125.6 ms).  A pair with a NaN distance is beyond
+// both cut-offs: without a CG-G0 term (CGG0: gdd is then not NaN) its force is
+// 0 times its axis, and where that is NaN too the clamp makes it -kMaxTerm.
+template <bool CGG0>
+__device__ __forceinline__ void couple_force(unsigned* f3, uint32_t c, uint32_t i, uint32_t j, float2 sx, float2 sy, float2 sz,
+                                             float2 gdd, float2 pg, float2 r)
 {
 	const float2 mg = f2s(kRoundMagic);
+	float2 gx = f2mul(sx, gdd), gy = f2mul(sy, gdd), gz = f2mul(sz, gdd);
 	const bool small = fabsf(pg.x) < 7.999f && fabsf(pg.y) < 7.999f;
 	if (!__all_sync(0xffffffffu, small)) {
+		if constexpr (!CGG0) {
+			gdd = f2(isnan(r.x) ? 0.0f : gdd.x, isnan(r.y) ? 0.0f : gdd.y);
+			gx = f2mul(sx, gdd); gy = f2mul(sy, gdd); gz = f2mul(sz, gdd);
+		}
 		gx = f2(clamp_term(gx.x), clamp_term(gx.y));
 		gy = f2(clamp_term(gy.x), clamp_term(gy.y));
 		gz = f2(clamp_term(gz.x), clamp_term(gz.y));
@@ -571,7 +587,9 @@ __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, i
 		// electrostatics and desolvation, cut-off 20.48 A
 		{
 			const float2 in20 = f2(lt1(r.x, 20.48f), lt1(r.y, 20.48f));
-			const float2 rr = f2(fmaxf(r.x, emd), fmaxf(r.y, emd));
+			// a NaN distance makes the energy NaN, as the reference's 0 * r of a
+			// pair that is no CG-G0 pair does
+			const float2 rr = CGG0 ? f2(fmaxf(r.x, emd), fmaxf(r.y, emd)) : f2(max_nan(r.x, emd), max_nan(r.y, emd));
 			const float2 ir = f2mul(inv_dist, f2s(inv_spacing));
 			const float2 inv_r = f2(fminf(ir.x, inv_emd), fminf(ir.y, inv_emd));
 			const float2 d2 = f2mul(rr, rr);
@@ -601,10 +619,12 @@ __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, i
 			// fixed-point forces; the 1024 scale folded into gdd (a power of two:
 			// the same rounding as quant(sub * gdd))
 			const float2 gdd = f2mul(pg, f2mul(inv_dist, f2s(-kTermScale)));
-			const float2 gx = f2mul(sx, gdd), gy = f2mul(sy, gdd), gz = f2mul(sz, gdd);
 			if constexpr (COUPLED) {
-				couple_force(reinterpret_cast<unsigned*>(f3), a1, a2, b2, gx, gy, gz, pg);
+				// (the vote's sizes: NaN with r)
+				const float2 size = CGG0 ? f2fma(f2s(0.0f), r, pg) : pg;
+				couple_force<CGG0>(reinterpret_cast<unsigned*>(f3), a1, a2, b2, sx, sy, sz, gdd, size, r);
 			} else {
+				const float2 gx = f2mul(sx, gdd), gy = f2mul(sy, gdd), gz = f2mul(sz, gdd);
 				pair_force(f3, a1, a2, gx.x, gy.x, gz.x);
 				pair_force(f3, b1, b2, gx.y, gy.y, gz.y);
 			}
@@ -632,8 +652,10 @@ template <int TPP, bool GRAD, bool TERMS = false>
 __device__ __forceinline__ float pair_terms(const LigDev& L, const PoseSmem& S, int rank, float* tsum = nullptr)
 {
 	if (!L.coupled) return pair_loop<TPP, GRAD, TERMS, false, true>(L, S, rank, tsum);
-	return L.cgg0 ? pair_loop<TPP, GRAD, TERMS, true, true>(L, S, rank, tsum)
-	              : pair_loop<TPP, GRAD, TERMS, true, false>(L, S, rank, tsum);
+	// (with TERMS a NaN distance shows in the CG-G0 sum alone)
+	if constexpr (TERMS) return pair_loop<TPP, GRAD, TERMS, true, true>(L, S, rank, tsum);
+	else return L.cgg0 ? pair_loop<TPP, GRAD, TERMS, true, true>(L, S, rank, tsum)
+	                   : pair_loop<TPP, GRAD, TERMS, true, false>(L, S, rank, tsum);
 }
 
 // Pairs with other exponents than 12-6 / 12-10 (modified pair potentials;
