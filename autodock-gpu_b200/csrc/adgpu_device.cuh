@@ -830,7 +830,9 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 		float4 t0, t1, e0, e1, d0, d1;
 		if constexpr (REF_GRID) {
 			const size_t g3 = (size_t)L.gx * L.gy * L.gz;
-			const size_t p = (size_t)xl + (size_t)yl * L.gx + (size_t)zl * L.gx * L.gy;
+			// (through int: a NaN coordinate passes the test above and is 0 as an
+			// int, but 2^63 as a size_t)
+			const size_t p = (size_t)(int)xl + (size_t)(int)yl * L.gx + (size_t)(int)zl * L.gx * L.gy;
 			const size_t M = (size_t)(L.rec_floats / 8 - 2);
 			const float4* tp = reinterpret_cast<const float4*>(L.grid + ((((size_t)slot - 2) * g3 + p) << 2));
 			const float4* ep = reinterpret_cast<const float4*>(L.grid + ((M * g3 + p) << 2));
