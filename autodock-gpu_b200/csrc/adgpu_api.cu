@@ -47,12 +47,12 @@ adgpu_status cuda_fail(cudaError_t e, const char* what)
 // ---------------------------------------------------------------------------
 constexpr int lga_min_ctas(int kind) { return kind >= 2 && kind <= 4 ? ADGPU_MIN_CTAS_GRAD : ADGPU_MIN_CTAS; }
 
-template <int TPP, int KIND, int SUMS>
+template <int TPP, int KIND, int SUMS, bool CGG0>
 __global__ void __launch_bounds__(128, lga_min_ctas(KIND)) lga_kernel(KArgs a, float* grads)
 {
 	if (a.stop_flag && *a.stop_flag) return;
 	int gid, ngroups;
-	Group<TPP> G;
+	Group<TPP, CGG0> G;
 	GroupSmem S;
 	group_of<TPP, SUMS>(a, gid, ngroups, G, S);
 	// Local searches run for a data-dependent number of iterations, so pose
@@ -173,13 +173,13 @@ __global__ void relayout_grid_kernel(const float* __restrict__ ref, float* __res
 // ---------------------------------------------------------------------------
 int g_num_sms = 0;
 
-template <int TPP, int KIND, int SUMS = TPP>
-adgpu_status launch_lga(const KArgs& a, float* grads, cudaStream_t stream, int cta_threads)
+template <int TPP, int KIND, int SUMS, bool CGG0>
+adgpu_status launch_lga_as(const KArgs& a, float* grads, cudaStream_t stream, int cta_threads)
 {
 	if (a.nblocks == 0) return ADGPU_OK;
 	const int gpc = cta_threads / TPP;
 	const int bytes = group_smem_bytes(a.L.natoms, a.L.ntors, (int)a.ref_threads, TPP, ep_records(a.L, TPP, SUMS)) * gpc;
-	auto kfn = lga_kernel<TPP, KIND, SUMS>;
+	auto kfn = lga_kernel<TPP, KIND, SUMS, CGG0>;
 	if (bytes > 48 * 1024) ADGPU_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "smem attribute");
 	static int carveout = -2;           // per instantiation: the last preference set
 	const int pct = smem_carveout_pct(bytes, lga_min_ctas(KIND));
@@ -200,6 +200,15 @@ adgpu_status launch_lga(const KArgs& a, float* grads, cudaStream_t stream, int c
 	kfn<<<grid, cta_threads, bytes, stream>>>(a, grads);
 	ADGPU_CUDA(cudaGetLastError(), "kernel launch");
 	return ADGPU_OK;
+}
+
+template <int TPP, int KIND, int SUMS = TPP>
+adgpu_status launch_lga(const KArgs& a, float* grads, cudaStream_t stream, int cta_threads)
+{
+	// (kind 8 adds up the CG-G0 terms anyway; ligands with CG-G0 pairs share no sums)
+	if constexpr (KIND != 8 && SUMS == TPP)
+		if (a.L.cgg0) return launch_lga_as<TPP, KIND, SUMS, true>(a, grads, stream, cta_threads);
+	return launch_lga_as<TPP, KIND, SUMS, false>(a, grads, stream, cta_threads);
 }
 
 // Threads per pose for a launch of n blocks when none is configured.
@@ -314,8 +323,9 @@ adgpu_status dock_resident(ApiState& s, int lsmet, uint32_t runs, uint64_t max_e
 	// once end together, so with AutoStop there is nothing to work ahead of.
 	// (36-atom ligand, 39 runs, B200, pipelined against synchronous: ADAM 35.9
 	// and 41.4 ms, FIRE 44.4 and 43.3; 5 runs 9.8 and 9.4, 12.8 and 10.9.)
-	const bool as_gains = as_frequency == 0 || lsmet < 2 ||
-	                      (lsmet == 2 && tasks > 4L * ADGPU_MIN_CTAS_GRAD * g_num_sms);
+	// Ligands with CG-G0 pairs have no pipelined kernels with AutoStop.
+	const bool as_gains = as_frequency == 0 || (!s.tables.dev.cgg0 &&
+	                      (lsmet < 2 || (lsmet == 2 && tasks > 4L * ADGPU_MIN_CTAS_GRAD * g_num_sms)));
 	if (s.pipeline && as_fits && as_gains && pipeline_applies(dp, runs)) {
 		*autostopped = 0;
 		KArgs base = make_args(s);

@@ -227,8 +227,16 @@ __device__ __forceinline__ void map_angle(float& a)
 // ---- pose group ------------------------------------------------------------------
 // TPP threads scoring one pose.  TPP == 32 is warp-synchronous; larger groups
 // sync with a named barrier (id 1 + group index within the CTA).
-template <int TPP>
+// CGG0: it scores ligands with CG-G0 pairs (flexible rings).  These have
+// kernels of their own, since a second pair loop beside the first one cost
+// every ligand instruction fetches (with it, without it and at the start of
+// both changes, dockings of 95 runs, B200: ADAM with 22 atoms and 1 torsion
+// 21.4, 20.4 and 20.9 ms, ADADELTA 21.1, 20.0 and 20.3; with 40 atoms and 10
+// torsions 63.4, 63.6 and 68.6 ms, 69.5, 69.2 and 71.9; a branch around the
+// term in the one loop 1.5 % more with 40 atoms).
+template <int TPP, bool CGG0 = false>
 struct Group {
+	static constexpr bool kCgg0 = CGG0;
 	int rank;          // 0..TPP-1
 	int bar_id;        // named barrier for TPP > 32
 	float* red;        // TPP/32 * 8 floats of scratch for cross-warp reductions
@@ -498,8 +506,8 @@ __device__ __forceinline__ void couple_force(unsigned* f3, uint32_t c, uint32_t 
 // TERMS (energy only): also adds this thread's vdW/H-bond, electrostatic,
 // desolvation and CG-G0 sums to tsum[0..3].
 // With COUPLED (the host's tables, L.coupled) the two pairs of a record share
-// their first atom: one position load and one set of atomics for it.  CGG0:
-// the ligand has CG-G0 pairs (flexible rings).
+// their first atom: one position load and one set of atomics for it.  Without
+// CGG0 the ligand has no CG-G0 pairs.
 // EP: each record's energies go to S.ep instead (pair_sum).
 template <int TPP, bool GRAD, bool TERMS, bool COUPLED, bool CGG0, bool EP = false>
 __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, int rank, float* tsum)
@@ -648,16 +656,6 @@ __device__ __forceinline__ float pair_sum(const LigDev& L, const PoseSmem& S, in
 	return esum.x + esum.y;
 }
 
-template <int TPP, bool GRAD, bool TERMS = false>
-__device__ __forceinline__ float pair_terms(const LigDev& L, const PoseSmem& S, int rank, float* tsum = nullptr)
-{
-	if (!L.coupled) return pair_loop<TPP, GRAD, TERMS, false, true>(L, S, rank, tsum);
-	// (with TERMS a NaN distance shows in the CG-G0 sum alone)
-	if constexpr (TERMS) return pair_loop<TPP, GRAD, TERMS, true, true>(L, S, rank, tsum);
-	else return L.cgg0 ? pair_loop<TPP, GRAD, TERMS, true, true>(L, S, rank, tsum)
-	                   : pair_loop<TPP, GRAD, TERMS, true, false>(L, S, rank, tsum);
-}
-
 // Pairs with other exponents than 12-6 / 12-10 (modified pair potentials;
 // the AD4 front end has none), one per thread, the reference's terms with
 // sd^-m and sd^-n by repeated squaring.
@@ -714,7 +712,7 @@ __device__ __forceinline__ float pair_terms_generic(const LigDev& L, const PoseS
 // records' energies, added up by the lower half, take at most 8 KB.
 __host__ __device__ inline bool shares_sums(const LigDev& L)
 {
-	return L.coupled && L.ngpairs == 0 && L.natoms <= 64 && L.npairs2 <= 1024;
+	return L.coupled && !L.cgg0 && L.ngpairs == 0 && L.natoms <= 64 && L.npairs2 <= 1024;
 }
 
 // ---- the scorer -----------------------------------------------------------------------
@@ -725,7 +723,8 @@ __host__ __device__ inline bool shares_sums(const LigDev& L)
 // the pose coordinates in S.
 // REF_GRID: L.grid is the reference's own layout (4 replicated floats per
 // point and map, host/src/processgrid.cpp:244-248) instead of cell records;
-// the same 8 corner values are read, from two 16-byte loads per map.
+// the same 8 corner values are read, from two 16-byte loads per map, and the
+// pairs are not coupled.
 // TERMS (energy only): terms[0..7] (written by rank 0) = intermolecular type
 // map, electrostatic and desolvation energies, intramolecular vdW/H-bond,
 // electrostatic, desolvation and CG-G0 energies, and the number of atoms
@@ -752,9 +751,9 @@ __host__ __device__ inline bool shares_sums(const LigDev& L)
 // is dealt out to threads, and a search of hundreds of steps on every bit of
 // them; SUMS 64 with 128 threads (shares_sums) gives what 64 threads give, in
 // the shorter time of 128.
-template <int TPP, bool GRAD, bool REF_GRID = false, bool TERMS = false, int SUMS = TPP>
+template <int TPP, bool GRAD, bool REF_GRID = false, bool TERMS = false, int SUMS = TPP, class GT>
 __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float* __restrict__ grad,
-                           const PoseSmem& S, const Group<TPP>& G, float* terms = nullptr)
+                           const PoseSmem& S, const GT& G, float* terms = nullptr)
 {
 	const int rank = G.rank;
 	// the upper half takes the lower half's intermolecular terms
@@ -931,12 +930,10 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 	}
 
 	// 4. intramolecular pairs (cuda/calcMergeEneGra.cu:418-602)
-	float e_pair, e_gen = 0.0f;
-	if constexpr (SUMS != TPP) {
-		e_pair = L.cgg0 ? pair_loop<TPP, GRAD, false, true, true, true>(L, S, rank, nullptr)
-		                : pair_loop<TPP, GRAD, false, true, false, true>(L, S, rank, nullptr);
-	} else if constexpr (TERMS) e_pair = pair_terms<TPP, GRAD, TERMS>(L, S, rank, tt + 3);
-	else e_pair = pair_terms<TPP, GRAD>(L, S, rank);
+	// (with TERMS, a NaN distance shows in the CG-G0 sum alone)
+	constexpr bool kCgg0 = GT::kCgg0 || TERMS || REF_GRID;
+	float e_gen = 0.0f;
+	float e_pair = pair_loop<TPP, GRAD, TERMS, !REF_GRID, kCgg0, SUMS != TPP>(L, S, rank, TERMS ? tt + 3 : nullptr);
 	if (L.ngpairs > 0) {
 		if constexpr (TERMS) e_gen = pair_terms_generic<TPP, GRAD, TERMS>(L, S, rank, tt + 3);
 		else e_gen = pair_terms_generic<TPP, GRAD>(L, S, rank);

@@ -214,8 +214,8 @@ __device__ bool take_task(const TickArgs& t, const TickClass& C, int lane, int w
 	return false;
 }
 
-template <int TPP>
-__device__ int group_isum(int v, const Group<TPP>& G, GroupHdr& H)
+template <int TPP, class GT>
+__device__ int group_isum(int v, const GT& G, GroupHdr& H)
 {
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -233,8 +233,8 @@ __device__ int group_isum(int v, const Group<TPP>& G, GroupHdr& H)
 }
 
 // Lowest energy of a run's population (smallest index on ties) -> best_e, best_g.
-template <int TPP>
-__device__ void best_of_run(const ReqDev& rq, int run, int c, int P, const Group<TPP>& G, GroupHdr& H)
+template <int TPP, class GT>
+__device__ void best_of_run(const ReqDev& rq, int run, int c, int P, const GT& G, GroupHdr& H)
 {
 	const float* E = rq.e[c] + (size_t)run * P;
 	float bv = FLT_MAX;
@@ -272,7 +272,7 @@ __device__ void open_phase(const TickArgs& t, const TickClass& C, const ReqDev& 
 	if ((int)(phase >> 1) >= t.runs[w].limit) atomicSub(&C.ctl->alive, 1);      // parked until the next tick
 }
 
-template <int TPP, int LSMET>
+template <int TPP, int LSMET, bool CGG0>
 __device__ void engine_worker(const TickArgs& t, const TickClass& C)
 {
 	extern __shared__ __align__(16) char smem[];
@@ -280,7 +280,7 @@ __device__ void engine_worker(const TickArgs& t, const TickClass& C)
 	char* base = smem + (size_t)local * C.group_bytes;
 	GroupHdr& H = *reinterpret_cast<GroupHdr*>(base);
 	char* scratch = base + kHdrBytes;
-	Group<TPP> G;
+	Group<TPP, CGG0> G;
 	G.rank = threadIdx.x % TPP;
 	G.bar_id = 1 + local;
 	G.red = nullptr;
@@ -412,13 +412,14 @@ __device__ void engine_worker(const TickArgs& t, const TickClass& C)
 }
 
 // One kernel per local search; its CTAs are split into three ranges, one per
-// threads-per-pose class, each range serving its class's runs.
-template <int LSMET>
+// threads-per-pose class, each range serving its class's runs.  CGG0: some
+// request's ligand has CG-G0 pairs (the others score the same bits with it).
+template <int LSMET, bool CGG0>
 __global__ void __launch_bounds__(kEngineThreads, ADGPU_ENGINE_MIN_CTAS) engine_kernel(const TickArgs t)
 {
-	if ((int)blockIdx.x < t.cls[0].cta_end) engine_worker<32, LSMET>(t, t.cls[0]);
-	else if ((int)blockIdx.x < t.cls[1].cta_end) engine_worker<64, LSMET>(t, t.cls[1]);
-	else engine_worker<128, LSMET>(t, t.cls[2]);
+	if ((int)blockIdx.x < t.cls[0].cta_end) engine_worker<32, LSMET, CGG0>(t, t.cls[0]);
+	else if ((int)blockIdx.x < t.cls[1].cta_end) engine_worker<64, LSMET, CGG0>(t, t.cls[1]);
+	else engine_worker<128, LSMET, CGG0>(t, t.cls[2]);
 }
 
 // Tick set-up and tear-down: each work item's phase counter from its run's
@@ -557,7 +558,7 @@ static size_t request_bytes(int runs, int pop, size_t tables)
 // class getting no more CTAs than its runs can keep busy at once.
 template <int LSMET>
 static adgpu_status launch_engine(Engine& E, TickArgs t, const int* nruns, const double* weight, const int* max_tasks,
-                                  const int* max_atoms, const int* max_tors)
+                                  const int* max_atoms, const int* max_tors, bool cgg0)
 {
 	static const int tpps[3] = {32, 64, 128};
 	int smem = 0;
@@ -565,7 +566,7 @@ static adgpu_status launch_engine(Engine& E, TickArgs t, const int* nruns, const
 		t.cls[k].group_bytes = kHdrBytes + group_smem_bytes(max_atoms[k], max_tors[k], 64, tpps[k]);
 		if (nruns[k]) smem = std::max(smem, t.cls[k].group_bytes * (kEngineThreads / tpps[k]));
 	}
-	auto kern = engine_kernel<LSMET>;
+	auto kern = cgg0 ? engine_kernel<LSMET, true> : engine_kernel<LSMET, false>;
 	if (smem > 48 * 1024) {
 		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 		if (e != cudaSuccess) return cuda_fail(e, "engine smem");
@@ -810,6 +811,7 @@ adgpu_status adgpu_engine_tick(adgpu_engine* en, int* completed)
 	std::vector<RunRef> work[NC];
 	int max_atoms[NC], max_tors[NC], max_tasks[NC];
 	double weight[NC];
+	bool cg[4] = {false, false, false, false};      // per local search: a ligand has CG-G0 pairs
 	for (int c = 0; c < NC; c++) { max_atoms[c] = 1; max_tors[c] = 0; max_tasks[c] = 1; weight[c] = 0; }
 	std::vector<uint32_t> wprio[NC];      // request rank by age (E.requests is ordered by id = admission)
 	for (auto& kv : E.requests) {
@@ -827,6 +829,7 @@ adgpu_status adgpu_engine_tick(adgpu_engine* en, int* completed)
 		max_atoms[cls] = std::max(max_atoms[cls], r.natoms);
 		max_tors[cls] = std::max(max_tors[cls], r.ntors);
 		max_tasks[cls] = std::max({max_tasks[cls], (int)dp.num_of_lsentities, dp.pop_size});
+		cg[r.dev.lsmet] |= r.dev.a.L.cgg0 != 0;
 		weight[cls] += (double)r.runs * (r.dev.a.L.npairs + 8.0 * r.natoms + 64.0);
 	}
 	if (completed) *completed = 0;
@@ -903,10 +906,10 @@ adgpu_status adgpu_engine_tick(adgpu_engine* en, int* completed)
 		if (!any) continue;
 		adgpu_status st = ADGPU_OK;
 		switch (m) {
-		case LS_SW: st = launch_engine<LS_SW>(E, t, nr, wt, mx, ma, mt); break;
-		case LS_AD: st = launch_engine<LS_AD>(E, t, nr, wt, mx, ma, mt); break;
-		case LS_ADAM: st = launch_engine<LS_ADAM>(E, t, nr, wt, mx, ma, mt); break;
-		default: st = launch_engine<LS_FIRE>(E, t, nr, wt, mx, ma, mt); break;
+		case LS_SW: st = launch_engine<LS_SW>(E, t, nr, wt, mx, ma, mt, cg[m]); break;
+		case LS_AD: st = launch_engine<LS_AD>(E, t, nr, wt, mx, ma, mt, cg[m]); break;
+		case LS_ADAM: st = launch_engine<LS_ADAM>(E, t, nr, wt, mx, ma, mt, cg[m]); break;
+		default: st = launch_engine<LS_FIRE>(E, t, nr, wt, mx, ma, mt, cg[m]); break;
 		}
 		if (st != ADGPU_OK) return st;
 	}

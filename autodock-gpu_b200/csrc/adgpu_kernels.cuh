@@ -128,8 +128,8 @@ __device__ __forceinline__ GroupSmem carve_group(char* base, int natoms, int nto
 }
 
 // The group of this thread and its scratch.
-template <int TPP, int SUMS = TPP>
-__device__ __forceinline__ void group_of(const KArgs& a, int& gid, int& ngroups, Group<TPP>& G, GroupSmem& S)
+template <int TPP, int SUMS = TPP, class GT>
+__device__ __forceinline__ void group_of(const KArgs& a, int& gid, int& ngroups, GT& G, GroupSmem& S)
 {
 	extern __shared__ __align__(16) char smem[];
 	const int gpc = blockDim.x / TPP;               // groups per CTA
@@ -145,8 +145,8 @@ __device__ __forceinline__ void group_of(const KArgs& a, int& gid, int& ngroups,
 
 // LS entity choice shared by every local search (e.g. cuda/kernel_ad.cu:116-127):
 // entity 0 (the elite) is searched only with probability lsearch_rate %.
-template <int TPP>
-__device__ __forceinline__ int ls_entity(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, class GT>
+__device__ __forceinline__ int ls_entity(const KArgs& a, uint32_t b, const GT& G, const GroupSmem& S)
 {
 	int ent = (int)(b % a.dp.num_of_lsentities);
 	if (ent == 0) {
@@ -168,8 +168,8 @@ __device__ __forceinline__ int ls_entity(const KArgs& a, uint32_t b, const Group
 // success/fail step-size proxy falls to 0.01 or after max_num_of_iters.
 // ADAM (cuda/kernel_adam.cu:55-396): bias-corrected, always max_num_of_iters.
 // ---------------------------------------------------------------------------
-template <int TPP, int METHOD, int SUMS = TPP, bool POLL = false>
-__device__ void gradient_ls_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int METHOD, int SUMS = TPP, bool POLL = false, class GT>
+__device__ void gradient_ls_block(const KArgs& a, const PopBufs& pb, uint32_t b, const GT& G, const GroupSmem& S)
 {
 	const int P = a.dp.pop_size, NG = a.dp.num_of_genes;
 	const int run = (int)(b / a.dp.num_of_lsentities);
@@ -251,8 +251,8 @@ __device__ void gradient_ls_block(const KArgs& a, const PopBufs& pb, uint32_t b,
 // FIRE (device/kernel_fire.cl:76-895): N_min 5, f_inc 1.2, f_dec 0.8,
 // alpha0 0.2, f_alpha 0.99, dt_max 10, dt0 = dt_max/3, stop at dt < 1e-6.
 // ---------------------------------------------------------------------------
-template <int TPP, int SUMS = TPP, bool POLL = false>
-__device__ void fire_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int SUMS = TPP, bool POLL = false, class GT>
+__device__ void fire_block(const KArgs& a, const PopBufs& pb, uint32_t b, const GT& G, const GroupSmem& S)
 {
 	const float DT_INC = 1.2f, DT_DEC = 0.8f, ALPHA_START = 0.2f, ALPHA_DEC = 0.99f, DT_MAX = 10.0f, DT_MIN = 1e-6f;
 	const int P = a.dp.pop_size, NG = a.dp.num_of_genes;
@@ -328,8 +328,8 @@ __device__ void fire_block(const KArgs& a, const PopBufs& pb, uint32_t b, const 
 // ---------------------------------------------------------------------------
 // Solis-Wets with SWAT3 step scaling (cuda/kernel3.cu:30-308).
 // ---------------------------------------------------------------------------
-template <int TPP, int SUMS = TPP, bool POLL = false>
-__device__ void sw_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int SUMS = TPP, bool POLL = false, class GT>
+__device__ void sw_block(const KArgs& a, const PopBufs& pb, uint32_t b, const GT& G, const GroupSmem& S)
 {
 	const int P = a.dp.pop_size, NG = a.dp.num_of_genes;
 	const uint32_t T = a.ref_threads;
@@ -422,8 +422,8 @@ __device__ __forceinline__ void warp_minimum2(int lane, float& v, int& k)
 	}
 }
 
-template <int TPP, int SUMS = TPP>
-__device__ void ga_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int SUMS = TPP, class GT>
+__device__ void ga_block(const KArgs& a, const PopBufs& pb, uint32_t b, const GT& G, const GroupSmem& S)
 {
 	const int P = a.dp.pop_size, NG = a.dp.num_of_genes;
 	const uint32_t T = a.ref_threads;
@@ -511,22 +511,22 @@ __device__ void ga_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Gr
 }
 
 // The blocks above on the launch's own population buffers.
-template <int TPP, int METHOD, int SUMS = TPP>
-__device__ __forceinline__ void gradient_ls_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int METHOD, int SUMS = TPP, class GT>
+__device__ __forceinline__ void gradient_ls_block(const KArgs& a, uint32_t b, const GT& G, const GroupSmem& S)
 { gradient_ls_block<TPP, METHOD, SUMS>(a, bufs_of(a), b, G, S); }
-template <int TPP, int SUMS = TPP>
-__device__ __forceinline__ void fire_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int SUMS = TPP, class GT>
+__device__ __forceinline__ void fire_block(const KArgs& a, uint32_t b, const GT& G, const GroupSmem& S)
 { fire_block<TPP, SUMS>(a, bufs_of(a), b, G, S); }
-template <int TPP, int SUMS = TPP>
-__device__ __forceinline__ void sw_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int SUMS = TPP, class GT>
+__device__ __forceinline__ void sw_block(const KArgs& a, uint32_t b, const GT& G, const GroupSmem& S)
 { sw_block<TPP, SUMS>(a, bufs_of(a), b, G, S); }
-template <int TPP, int SUMS = TPP>
-__device__ __forceinline__ void ga_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int SUMS = TPP, class GT>
+__device__ __forceinline__ void ga_block(const KArgs& a, uint32_t b, const GT& G, const GroupSmem& S)
 { ga_block<TPP, SUMS>(a, bufs_of(a), b, G, S); }
 
 // Initial population energies (cuda/kernel1.cu:26-55).
-template <int TPP, int SUMS = TPP>
-__device__ void initpop_block(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int SUMS = TPP, class GT>
+__device__ void initpop_block(const KArgs& a, const PopBufs& pb, uint32_t b, const GT& G, const GroupSmem& S)
 {
 	const int NG = a.dp.num_of_genes;
 	for (int k = G.rank; k < NG; k += TPP) S.gen[k] = pb.conf[(size_t)b * kGenotypeStride + k];
@@ -536,14 +536,14 @@ __device__ void initpop_block(const KArgs& a, const PopBufs& pb, uint32_t b, con
 	G.sync();
 }
 
-template <int TPP, int SUMS = TPP>
-__device__ __forceinline__ void initpop_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int SUMS = TPP, class GT>
+__device__ __forceinline__ void initpop_block(const KArgs& a, uint32_t b, const GT& G, const GroupSmem& S)
 { initpop_block<TPP, SUMS>(a, bufs_of(a), b, G, S); }
 
 // Stand-alone scorer: energies (and gradients when a.conf_cur != nullptr is
 // used as the gradient output) of nblocks genotypes.
-template <int TPP, bool GRAD, int SUMS = TPP>
-__device__ void score_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S, float* grads)
+template <int TPP, bool GRAD, int SUMS = TPP, class GT>
+__device__ void score_block(const KArgs& a, uint32_t b, const GT& G, const GroupSmem& S, float* grads)
 {
 	const int NG = a.dp.num_of_genes;
 	for (int k = G.rank; k < NG; k += TPP) S.gen[k] = a.conf[(size_t)b * kGenotypeStride + k];
@@ -557,8 +557,8 @@ __device__ void score_block(const KArgs& a, uint32_t b, const Group<TPP>& G, con
 
 // The scorer's energy terms (energy only) of nblocks genotypes: a.e[b] the
 // energy, out[8b .. 8b+7] the terms (score_pose with TERMS).
-template <int TPP>
-__device__ void score_terms_block(const KArgs& a, uint32_t b, const Group<TPP>& G, const GroupSmem& S, float* out)
+template <int TPP, class GT>
+__device__ void score_terms_block(const KArgs& a, uint32_t b, const GT& G, const GroupSmem& S, float* out)
 {
 	const int NG = a.dp.num_of_genes;
 	for (int k = G.rank; k < NG; k += TPP) S.gen[k] = a.conf[(size_t)b * kGenotypeStride + k];

@@ -163,8 +163,8 @@ __device__ void pipe_try_start(const PipeArgs& p, int r)
 // entity only sends the scan round again.  Returns run << 11 | entity and the
 // generation in *gen, or -1 once every run has retired (or after idle_ns with
 // nothing to take: an error).
-template <int TPP>
-__device__ int pipe_take(const PipeArgs& p, int worker, const Group<TPP>& G, int* gen)
+template <class GT>
+__device__ int pipe_take(const PipeArgs& p, int worker, const GT& G, int* gen)
 {
 	volatile PipeCtl* vc = p.ctl;
 	const int lane = G.rank;            // called by the group's first warp only
@@ -210,15 +210,15 @@ __device__ int pipe_take(const PipeArgs& p, int worker, const Group<TPP>& G, int
 }
 
 // The GA step of a task; GA_TPP < TPP: by the group's first warp.
-template <int TPP, int GA_TPP, int SUMS>
-__device__ __forceinline__ void pipe_ga(const KArgs& a, const PopBufs& pb, uint32_t b, const Group<TPP>& G, const GroupSmem& S)
+template <int TPP, int GA_TPP, int SUMS, class GT>
+__device__ __forceinline__ void pipe_ga(const KArgs& a, const PopBufs& pb, uint32_t b, const GT& G, const GroupSmem& S)
 {
 	if constexpr (GA_TPP == TPP) {
 		ga_block<TPP, SUMS>(a, pb, b, G, S);
 	} else {
 		static_assert(GA_TPP == 32, "the GA step takes the whole group or its first warp");
 		if (G.rank < 32) {
-			Group<32> W;
+			Group<32, GT::kCgg0> W;
 			W.rank = G.rank;
 			W.bar_id = G.bar_id;
 			W.red = G.red;
@@ -230,7 +230,7 @@ __device__ __forceinline__ void pipe_ga(const KArgs& a, const PopBufs& pb, uint3
 
 // AS: a docking with AutoStop (its own instantiation: the test's code in the
 // kernel of a docking without it cost that one 4 %).
-template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS>
+template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS, bool CGG0>
 __device__ void pipe_worker(const PipeArgs& p)
 {
 	extern __shared__ __align__(16) char smem[];
@@ -239,7 +239,7 @@ __device__ void pipe_worker(const PipeArgs& p)
 	PipeHdr& H = *reinterpret_cast<PipeHdr*>(base);
 	const LigDev& L0 = p.ka.L;
 	const GroupSmem S = carve_group(base + kPipeHdrBytes, L0.natoms, L0.ntors, 64, TPP, ep_records(L0, TPP, SUMS));
-	Group<TPP> G;
+	Group<TPP, CGG0> G;
 	G.rank = threadIdx.x % TPP;
 	G.bar_id = 1 + local;
 	G.red = S.red;
@@ -250,7 +250,7 @@ __device__ void pipe_worker(const PipeArgs& p)
 		if (G.rank < 32) {
 			if (G.rank == 0 && H.t_task) H.busy += (unsigned long long)(global_ns() - H.t_task);
 			int gen = 0;
-			const int task = pipe_take<TPP>(p, worker, G, &gen);
+			const int task = pipe_take(p, worker, G, &gen);
 			if (G.rank == 0) {
 				H.task = task;
 				H.t_task = task >= 0 ? global_ns() : 0;
@@ -393,10 +393,10 @@ __device__ void pipe_worker(const PipeArgs& p)
 
 constexpr int pipe_min_ctas(int lsmet) { return lsmet == LS_SW ? ADGPU_PIPE_MIN_CTAS_SW : ADGPU_PIPE_MIN_CTAS; }
 
-template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS>
+template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS, bool CGG0>
 __global__ void __launch_bounds__(kPipeThreads, pipe_min_ctas(LSMET)) pipe_kernel(const PipeArgs p)
 {
-	pipe_worker<TPP, LSMET, GA_TPP, AS, SUMS>(p);
+	pipe_worker<TPP, LSMET, GA_TPP, AS, SUMS, CGG0>(p);
 }
 
 // Check 0 (before the first generation) and the first generation's GA tasks.
@@ -466,10 +466,10 @@ __global__ void __launch_bounds__(256) pipe_final_kernel(PipeArgs p, long long* 
 // Initial check and tasks, the persistent launch, the final accounting; the
 // grid is sized from the kernel's occupancy (persistent: every pose group a
 // worker) and capped by the entities a generation offers.
-template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS>
+template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS, bool CGG0>
 static adgpu_status launch_pipe_as(PipeArgs p, long long* d_out, cudaStream_t st)
 {
-	auto kfn = pipe_kernel<TPP, LSMET, GA_TPP, AS, SUMS>;
+	auto kfn = pipe_kernel<TPP, LSMET, GA_TPP, AS, SUMS, CGG0>;
 	const int gpc = kPipeThreads / TPP;
 	const int bytes = p.group_bytes * gpc;
 	if (bytes > 48 * 1024) ADGPU_CUDA_RET(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "pipeline smem");
@@ -495,8 +495,10 @@ static adgpu_status launch_pipe_as(PipeArgs p, long long* d_out, cudaStream_t st
 template <int TPP, int LSMET, int GA_TPP = TPP, int SUMS = TPP>
 static adgpu_status launch_pipe(const PipeArgs& p, long long* d_out, cudaStream_t st)
 {
-	if (p.as_state) return launch_pipe_as<TPP, LSMET, GA_TPP, true, SUMS>(p, d_out, st);
-	if constexpr (GA_TPP == TPP && SUMS == TPP) return launch_pipe_as<TPP, LSMET, GA_TPP, false, SUMS>(p, d_out, st);
+	if (p.as_state) return launch_pipe_as<TPP, LSMET, GA_TPP, true, SUMS, false>(p, d_out, st);
+	if constexpr (GA_TPP == TPP && SUMS == TPP)
+		return p.ka.L.cgg0 ? launch_pipe_as<TPP, LSMET, GA_TPP, false, SUMS, true>(p, d_out, st)
+		                   : launch_pipe_as<TPP, LSMET, GA_TPP, false, SUMS, false>(p, d_out, st);
 	else return fail(ADGPU_ERR_ARG, "GA group size");
 }
 
@@ -548,6 +550,7 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 	if (!pipeline_applies(dp, runs)) return fail(ADGPU_ERR_ARG, "pipelined docking needs a 100 % local-search rate");
 	if (tpp == 0) tpp = pipeline_default_tpp(lsmet, (long)runs * dp.pop_size);
 	if (tpp != 32 && tpp != 64 && tpp != 128) return fail(ADGPU_ERR_ARG, "threads per pose must be 32, 64 or 128");
+	if (as.frequency && base.L.cgg0) return fail(ADGPU_ERR_ARG, "pipelined AutoStop of a ligand with CG-G0 pairs");
 	const int ga_tpp = as.frequency ? as.ga_tpp : tpp;
 	if (ga_tpp != tpp && (ga_tpp != 32 || tpp != 64)) return fail(ADGPU_ERR_ARG, "GA group size");
 	// 128 threads with the sums of 64: a docking that leaves SMs short of work
