@@ -761,6 +761,14 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 	static_assert(SUMS == TPP || (SUMS == 64 && kCanSplit), "sums of another group size");
 	const bool split = kCanSplit && (SUMS != TPP || (GRAD && L.natoms <= TPP / 2));
 
+	// Torsion chains are read four ids a word, but byte by byte in the
+	// no-allocation tables, where they are not aligned, and by groups of several
+	// warps without gradients, for which the word's load ahead of the chain is
+	// the longer way (Solis-Wets, B200: docking of one 32-atom run at 128 threads
+	// 10.8 and 10.1 ms, launches of 450 40-atom entities at 64 threads 11.0 and
+	// 10.3; at 32 threads 95 runs of a 22-atom ligand 10.4 and 10.7).
+	constexpr bool kWords = !REF_GRID && (GRAD || TPP == 32);
+
 	// 0. this thread's first atom (with split, the upper half's: its partner's)
 	struct AtomIn { float4 r; uint32_t info, chain; int len; };
 	auto load_atom = [&](int a) {
@@ -768,8 +776,8 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 		x.r = L.atom_xyzq[a];
 		x.info = L.atom_info[a];
 		x.len = L.chain_len[a];
-		x.chain = 0;                      // four torsion ids a word (single bytes in the no-allocation tables)
-		if constexpr (!REF_GRID) {
+		x.chain = 0;                      // four torsion ids a word
+		if constexpr (kWords) {
 			if (x.len > 0) x.chain = __ldg(reinterpret_cast<const uint32_t*>(L.chain + (x.info >> 16)));
 		}
 		return x;
@@ -878,7 +886,7 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 		const int cs = in.info >> 16;
 		uint32_t next = in.chain;
 		for (int i = 0; i < in.len; i++) {
-			if constexpr (REF_GRID) next = L.chain[cs + i];
+			if constexpr (!kWords) next = L.chain[cs + i];
 			else if (i > 0) next = (i & 3) ? next >> 8 : __ldg(reinterpret_cast<const uint32_t*>(L.chain + cs + i));
 			const int k = (int)(next & 0xFFu);
 			float4 m4 = L.tors_mv[k];
