@@ -49,24 +49,24 @@ struct PopBufs {
 __device__ __forceinline__ PopBufs bufs_of(const KArgs& a) { return PopBufs{a.conf_cur, a.e_cur, a.conf, a.e, 0}; }
 
 // In the pipelined docking loop a search of a generation past the stop is
-// worked on for nothing, and the docking ends only when it does.  So every
-// eighth iteration (every 32nd with several warps per pose, where a poll is
-// part of the chain of an evaluation) the stop is read ahead of a scoring,
-// which hides the load, thread 0's answer goes through S.misc ahead of a
-// barrier, and after the barrier the whole group leaves.  B200, dockings of
+// worked on for nothing, and the docking ends only when it does.  So at the end
+// of every eighth iteration (every 32nd with several warps per pose, where a
+// poll is part of the chain of an evaluation) thread 0 reads the stop, its
+// answer goes through S.misc, and the whole group leaves.  B200, dockings of
 // 100 runs: Solis-Wets 82.4 -> 79.1 ms (7 generations), ADADELTA 122.9 ->
 // 120.7 (30), 50 runs of ADAM with flexible residues 73.7 -> 70.6 (4).
 // POLL: a search of the pipelined loop (in the others the code alone cost a
 // Solis-Wets launch of 64 threads per pose 3 %).
-template <int TPP, bool POLL>
-__device__ __forceinline__ bool polls_abandon(uint32_t it)
+template <int TPP, bool POLL, class GT>
+__device__ __forceinline__ bool abandoned(const KArgs& a, const PopBufs& pb, uint32_t it, const GT& G, int* misc)
 {
-	return POLL && (it & (TPP == 32 ? 7u : 31u)) == 0;
-}
-__device__ __forceinline__ int read_abandon(const KArgs& a) { return *reinterpret_cast<const volatile int*>(a.abandon); }
-__device__ __forceinline__ void post_abandon(const PopBufs& pb, int rank, int* misc, int stop)
-{
-	if (rank == 0) misc[14] = stop >= 0 && stop <= pb.gen;
+	if (!POLL || (it & (TPP == 32 ? 7u : 31u)) != 0) return false;
+	if (G.rank == 0) {
+		const int stop = *reinterpret_cast<const volatile int*>(a.abandon);
+		misc[14] = stop >= 0 && stop <= pb.gen;
+	}
+	G.sync();
+	return misc[14] != 0;
 }
 
 // Pair records whose energies a group of tpp threads with the sums of `sums`
@@ -195,11 +195,7 @@ __device__ void gradient_ls_block(const KArgs& a, const PopBufs& pb, uint32_t b,
 			b1r = 1.0f - powf(a.dp.adam_beta1, t);
 			b2r = 1.0f - powf(a.dp.adam_beta2, t);
 		}
-		const bool poll = polls_abandon<TPP, POLL>(it);
-		int stop = -1;
-		if (poll) stop = read_abandon(a);
 		const float energy = score_pose<TPP, true, false, false, SUMS>(a.L, S.gen, S.grad, S.pose, G);
-		if (poll) post_abandon(pb, G.rank, S.misc, stop);
 		float b1p = 0.f, b2p = 0.f;
 		if (METHOD == LS_ADAM) {
 			b1p = __shfl_sync(0xffffffffu, b1r, (int)(it & 31u));
@@ -232,7 +228,7 @@ __device__ void gradient_ls_block(const KArgs& a, const PopBufs& pb, uint32_t b,
 			if (energy < best_e) best_e = energy;
 		}
 		G.sync();
-		if (poll && S.misc[14]) return;
+		if (abandoned<TPP, POLL>(a, pb, it, G, S.misc)) return;
 	} while (it < a.dp.max_num_of_iters && (METHOD == LS_ADAM || rho > 0.01f));
 	float* dst = pb.conf + idx * kGenotypeStride;
 	for (int k = G.rank; k < NG; k += TPP) {
@@ -281,11 +277,7 @@ __device__ void fire_block(const KArgs& a, const PopBufs& pb, uint32_t b, const 
 	do {
 		for (int k = G.rank; k < NG; k += TPP) cgen[k] = gen[k] + dt * vel[k];
 		G.sync();
-		const bool poll = polls_abandon<TPP, POLL>(it);
-		int stop = -1;
-		if (poll) stop = read_abandon(a);
 		const float ce = score_pose<TPP, true, false, false, SUMS>(a.L, cgen, cgrad, S.pose, G);
-		if (poll) post_abandon(pb, G.rank, S.misc, stop);
 		float pw = 0.f;
 		for (int k = G.rank; k < NG; k += TPP) pw += -cgrad[k] * vel[k];
 		const float power = G.sum(pw);
@@ -313,7 +305,7 @@ __device__ void fire_block(const KArgs& a, const PopBufs& pb, uint32_t b, const 
 			for (int k = G.rank; k < NG; k += TPP) best[k] = gen[k];
 		}
 		G.sync();
-		if (poll && S.misc[14]) return;
+		if (abandoned<TPP, POLL>(a, pb, it, G, S.misc)) return;
 	} while (it < a.dp.max_num_of_iters && dt > DT_MIN);
 	float* dst = pb.conf + idx * kGenotypeStride;
 	for (int k = G.rank; k < NG; k += TPP) {
@@ -364,11 +356,7 @@ __device__ void sw_block(const KArgs& a, const PopBufs& pb, uint32_t b, const GT
 		G.sync();
 		for (int k = gs + G.rank; k < NG; k += TPP) cand[k] = gen[k] + dev[k] + bias[k];
 		G.sync();
-		const bool poll = polls_abandon<TPP, POLL>((uint32_t)iters);
-		int stop = -1;
-		if (poll) stop = read_abandon(a);
 		float ce = score_pose<TPP, false, false, false, SUMS>(a.L, cand, nullptr, S.pose, G);
-		if (poll) post_abandon(pb, G.rank, S.misc, stop);
 		evals++;
 		if (ce < cur_e) {
 			for (int k = gs + G.rank; k < NG; k += TPP) { gen[k] = cand[k]; bias[k] = 0.6f * bias[k] + 0.4f * dev[k]; }
@@ -390,7 +378,7 @@ __device__ void sw_block(const KArgs& a, const PopBufs& pb, uint32_t b, const GT
 		if (succ >= (int)a.dp.cons_limit) { rho *= 2.0f; succ = 0; }
 		else if (fail >= (int)a.dp.cons_limit) { rho *= 0.5f; fail = 0; }
 		G.sync();
-		if (poll && S.misc[14]) return;
+		if (abandoned<TPP, POLL>(a, pb, (uint32_t)iters, G, S.misc)) return;
 	}
 	float* dst = pb.conf + idx * kGenotypeStride;
 	for (int k = gs + G.rank; k < NG; k += TPP) {
