@@ -922,19 +922,27 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 			}
 		}
 	}
+	// a torsion's axis: unit vector and first atom
+	auto axis = [&](int k, float4& u, float4& e) {
+		const int2 ends = L.tors_ends[k];
+		const float3 e0 = ld3(S.xyz + 3 * ends.x), e1 = ld3(S.xyz + 3 * ends.y);
+		const float ux = e1.x - e0.x, uy = e1.y - e0.y, uz = e1.z - e0.z;
+		const float l = rnorm3df(ux, uy, uz);
+		u = make_float4(ux * l, uy * l, uz * l, 0.0f);
+		e = make_float4(e0.x, e0.y, e0.z, 0.0f);
+	};
+	// One warp that takes its torsion items in one round makes each item's axis
+	// there; with more rounds or warps the axes are made once per torsion.
+	// (B200, 95 runs, made once and per item: ADAM, 22 atoms and 4 torsions, 24.1
+	// and 23.6 ms, ADADELTA 23.1 and 22.7, 40,000 gradients of 40 atoms and 1
+	// torsion 116.2 and 114.9 us; of two rounds per item no better, and all of 40
+	// atoms and 10 torsions' 5 rounds per item cost 3 to 5 %.)
+	const bool item_axes = TPP == 32 && L.ntoritems <= 32;
 	if constexpr (GRAD) {
-		// the torsions' axes for step 6, once per torsion, in place of their
-		// quaternions (which every atom has used): unit vector and first atom.
-		// The last warp takes them: it has no more pairs than the others.
-		for (int k = TPP - 1 - rank; k < L.ntors; k += TPP) {
-			const int2 ends = L.tors_ends[k];
-			const float3 e0 = ld3(S.xyz + 3 * ends.x), e1 = ld3(S.xyz + 3 * ends.y);
-			float ux = e1.x - e0.x, uy = e1.y - e0.y, uz = e1.z - e0.z;
-			const float l = rnorm3df(ux, uy, uz);
-			ux *= l; uy *= l; uz *= l;
-			S.tq[k] = make_float4(ux, uy, uz, 0.0f);
-			S.tq[L.ntors + k] = make_float4(e0.x, e0.y, e0.z, 0.0f);
-		}
+		// for step 6, in place of the torsions' quaternions (which every atom has
+		// used).  The last warp takes them: it has no more pairs than the others.
+		if (!item_axes)
+			for (int k = TPP - 1 - rank; k < L.ntors; k += TPP) axis(k, S.tq[k], S.tq[L.ntors + k]);
 	}
 
 	// 4. intramolecular pairs (cuda/calcMergeEneGra.cu:418-602)
@@ -1040,15 +1048,26 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 	if constexpr (TPP == 32) G.sync();     // the forces of step 5 (larger groups: the barrier in the sum)
 	const bool last_only = TPP == 128 && ntoritems <= 96;
 	const int it0 = last_only ? (rank >= 96 ? rank - 96 : ntoritems) : (rank + 32) & (TPP - 1);
-	for (int it = it0; it < ntoritems; it += last_only ? 32 : TPP) {
-		const uint32_t item = __ldg(tor_items + it);
+	auto torsion_item = [&](uint32_t item, const float4& u, const float4& e0) {
 		const int k = item >> 8, la = item & 0xFF;
-		const float4 u = S.tq[k], e0 = S.tq[ntors + k];
 		const float3 pl = ld3(S.xyz + 3 * la), f = ld3(ff + 3 * la);
 		float3 r = make_float3(pl.x - e0.x, pl.y - e0.y, pl.z - e0.z);
 		float3 t = cross3(r, f);
 		float on_axis = (u.x * t.x + u.y * t.y + u.z * t.z) * spacing;
 		atomicAdd(&S.gg[6 + k], quant(on_axis * kDegToRad));
+	};
+	if (item_axes) {
+		if (rank < ntoritems) {
+			const uint32_t item = __ldg(tor_items + rank);
+			float4 u, e0;
+			axis(item >> 8, u, e0);
+			torsion_item(item, u, e0);
+		}
+	} else {
+		for (int it = it0; it < ntoritems; it += last_only ? 32 : TPP) {
+			const uint32_t item = __ldg(tor_items + it);
+			torsion_item(item, S.tq[item >> 8], S.tq[ntors + (item >> 8)]);
+		}
 	}
 	const int ngenes = L.ngenes;
 	G.sync();
