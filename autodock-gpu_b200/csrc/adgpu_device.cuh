@@ -234,9 +234,14 @@ __device__ __forceinline__ void map_angle(float& a)
 // 21.4, 20.4 and 20.9 ms, ADADELTA 21.1, 20.0 and 20.3; with 40 atoms and 10
 // torsions 63.4, 63.6 and 68.6 ms, 69.5, 69.2 and 71.9; a branch around the
 // term in the one loop 1.5 % more with 40 atoms).
-template <int TPP, bool CGG0 = false>
+// AHEAD: the pair loop loads a step's record during the step before, which
+// takes registers.  Groups of 128 threads score few poses per SM, so a step's
+// latency counts.  (With 64 threads it lost 2 to 4 %; without gradients the
+// Solis-Wets kernels' 72 registers do not hold it.)
+template <int TPP, bool CGG0 = false, bool AHEAD = TPP == 128>
 struct Group {
 	static constexpr bool kCgg0 = CGG0;
+	static constexpr bool kAhead = AHEAD;
 	int rank;          // 0..TPP-1
 	int bar_id;        // named barrier for TPP > 32
 	float* red;        // TPP/32 * 8 floats of scratch for cross-warp reductions
@@ -509,7 +514,8 @@ __device__ __forceinline__ void couple_force(unsigned* f3, uint32_t c, uint32_t 
 // their first atom: one position load and one set of atomics for it.  Without
 // CGG0 the ligand has no CG-G0 pairs.
 // EP: each record's energies go to S.ep instead (pair_sum).
-template <int TPP, bool GRAD, bool TERMS, bool COUPLED, bool CGG0, bool EP = false>
+// AHEAD: see Group.
+template <int TPP, bool GRAD, bool TERMS, bool COUPLED, bool CGG0, bool EP, bool AHEAD>
 __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, int rank, float* tsum)
 {
 	// loop invariants read once: when L lives in shared memory (the engine's
@@ -528,11 +534,7 @@ __device__ __forceinline__ float pair_loop(const LigDev& L, const PoseSmem& S, i
 	constexpr int kBlock = (int)pair2_block(COUPLED);
 	const float4* pr = L.pairs2 + (rank / 32) * kBlock + (rank % 32);
 	const uint32_t* pw = reinterpret_cast<const uint32_t*>(L.pairs2 + (rank / 32) * kBlock + 96) + (rank % 32);
-	// Groups of 128 load a step's record during the step before: they score
-	// few poses per SM, so a step's latency counts, and they have the registers.
-	// (With 64 threads it lost 2 to 4 %; without gradients the Solis-Wets
-	// kernels' 72 registers do not hold it.)
-	constexpr bool kAhead = TPP == 128 && GRAD;
+	constexpr bool kAhead = AHEAD && GRAD;
 	uint32_t wa = 0, wb = 0;
 	float4 q0, q1, q2;
 	q0 = q1 = q2 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -949,7 +951,7 @@ __device__ float score_pose(const LigDev& L, const float* __restrict__ g, float*
 	// (with TERMS, a NaN distance shows in the CG-G0 sum alone)
 	constexpr bool kCgg0 = GT::kCgg0 || TERMS || REF_GRID;
 	float e_gen = 0.0f;
-	float e_pair = pair_loop<TPP, GRAD, TERMS, !REF_GRID, kCgg0, SUMS != TPP>(L, S, rank, TERMS ? tt + 3 : nullptr);
+	float e_pair = pair_loop<TPP, GRAD, TERMS, !REF_GRID, kCgg0, SUMS != TPP, GT::kAhead>(L, S, rank, TERMS ? tt + 3 : nullptr);
 	if (L.ngpairs > 0) {
 		if constexpr (TERMS) e_gen = pair_terms_generic<TPP, GRAD, TERMS>(L, S, rank, tt + 3);
 		else e_gen = pair_terms_generic<TPP, GRAD>(L, S, rank);

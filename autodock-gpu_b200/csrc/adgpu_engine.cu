@@ -280,7 +280,9 @@ __device__ void engine_worker(const TickArgs& t, const TickClass& C)
 	char* base = smem + (size_t)local * C.group_bytes;
 	GroupHdr& H = *reinterpret_cast<GroupHdr*>(base);
 	char* scratch = base + kHdrBytes;
-	Group<TPP, CGG0> G;
+	// (no records ahead: one kernel holds the three group sizes, and the 128-thread
+	// one's registers would make the others spill)
+	Group<TPP, CGG0, false> G;
 	G.rank = threadIdx.x % TPP;
 	G.bar_id = 1 + local;
 	G.red = nullptr;
