@@ -393,8 +393,23 @@ __device__ void pipe_worker(const PipeArgs& p)
 
 constexpr int pipe_min_ctas(int lsmet) { return lsmet == LS_SW ? ADGPU_PIPE_MIN_CTAS_SW : ADGPU_PIPE_MIN_CTAS; }
 
-template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS, bool CGG0>
-__global__ void __launch_bounds__(kPipeThreads, pipe_min_ctas(LSMET)) pipe_kernel(const PipeArgs p)
+// Solis-Wets with 128 threads per pose: few runs wait for one evaluation after
+// another, and the 72 registers of 7 CTAs lengthen it; more runs want the CTAs.
+// 5 CTAs up to three entities a CTA of theirs (14 runs of 150; B200, 7 and 5
+// CTAs: one run of 11, 24 and 40 atoms 5.73 and 5.53, 6.84 and 6.46, 7.20 and
+// 6.85 ms, 12 runs 6.92 and 6.78, 9.39 and 9.19, 11.77 and 11.43, 16 runs 7.52
+// and 7.45, 10.36 and 10.32, 13.45 and 13.33, 20 runs 8.19 and 8.61, 11.50 and
+// 12.05, 15.50 and 15.67).
+constexpr int kFewCtasSw = 5;
+static bool few_entities(const PipeArgs& p)
+{
+	int dev = 0, sms = 0;
+	return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+	       (long)p.runs * p.pop <= 3L * kFewCtasSw * sms;
+}
+
+template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS, bool CGG0, int CTAS>
+__global__ void __launch_bounds__(kPipeThreads, CTAS) pipe_kernel(const PipeArgs p)
 {
 	pipe_worker<TPP, LSMET, GA_TPP, AS, SUMS, CGG0>(p);
 }
@@ -466,14 +481,14 @@ __global__ void __launch_bounds__(256) pipe_final_kernel(PipeArgs p, long long* 
 // Initial check and tasks, the persistent launch, the final accounting; the
 // grid is sized from the kernel's occupancy (persistent: every pose group a
 // worker) and capped by the entities a generation offers.
-template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS, bool CGG0>
+template <int TPP, int LSMET, int GA_TPP, bool AS, int SUMS, bool CGG0, int CTAS = pipe_min_ctas(LSMET)>
 static adgpu_status launch_pipe_as(PipeArgs p, long long* d_out, cudaStream_t st)
 {
-	auto kfn = pipe_kernel<TPP, LSMET, GA_TPP, AS, SUMS, CGG0>;
+	auto kfn = pipe_kernel<TPP, LSMET, GA_TPP, AS, SUMS, CGG0, CTAS>;
 	const int gpc = kPipeThreads / TPP;
 	const int bytes = p.group_bytes * gpc;
 	if (bytes > 48 * 1024) ADGPU_CUDA_RET(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "pipeline smem");
-	const int pct = smem_carveout_pct(bytes, pipe_min_ctas(LSMET));
+	const int pct = smem_carveout_pct(bytes, CTAS);
 	if (pct >= 0) ADGPU_CUDA_RET(cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, pct), "pipeline carveout");
 	int per_sm = 0, dev = 0, sms = 0;
 	ADGPU_CUDA_RET(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kPipeThreads, bytes), "pipeline occupancy");
@@ -496,6 +511,8 @@ template <int TPP, int LSMET, int GA_TPP = TPP, int SUMS = TPP>
 static adgpu_status launch_pipe(const PipeArgs& p, long long* d_out, cudaStream_t st)
 {
 	if (p.as_state) return launch_pipe_as<TPP, LSMET, GA_TPP, true, SUMS, false>(p, d_out, st);
+	if constexpr (TPP == 128 && LSMET == LS_SW)
+		if (!p.ka.L.cgg0 && few_entities(p)) return launch_pipe_as<TPP, LSMET, GA_TPP, false, SUMS, false, kFewCtasSw>(p, d_out, st);
 	if constexpr (GA_TPP == TPP && SUMS == TPP)
 		return p.ka.L.cgg0 ? launch_pipe_as<TPP, LSMET, GA_TPP, false, SUMS, true>(p, d_out, st)
 		                   : launch_pipe_as<TPP, LSMET, GA_TPP, false, SUMS, false>(p, d_out, st);
