@@ -36,14 +36,18 @@
 // population and PRNG states (local-search entity l of run r uses the states
 // of GA block r*P + l, inside its own run, because the local-search rate is
 // 100 %), so populations, energies and evaluation counts are bit-identical
-// to the generation-synchronous loop; only the PRNG states and the per-entity
-// evaluation counters of the discarded generations differ.
+// to the generation-synchronous loop; without AutoStop, only the PRNG states
+// and the per-entity evaluation counters are those that the discarded
+// generations left.
 //
 // AutoStop (the reference's default) is part of check g where as_frequency
 // divides g: the pose group that takes the check runs it on the energies that
 // generation g-1 left, whose buffer no generation overwrites before the check
 // is published, while the other groups work ahead.  Checks are published in
-// order: a later one waits (bounded) for the one before it.  The synchronous
+// order: a later one waits (bounded) for the one before it.  A docking with
+// AutoStop leaves the PRNG states and the evaluation counters of its last
+// generation too: each task first keeps its entity's (PipeKeep), and the ones
+// that discarded generations changed are put back.  The synchronous
 // loop ends each generation with its longest searches running alone (36-atom
 // ligand, 20 runs, ADADELTA, 64 threads per pose, B200: 90.3 ms a docking; this
 // loop with the same scorer 75.1 ms, the same final populations).
@@ -92,6 +96,14 @@ struct PipeCtl {
 	int fin[kPipeBufs];                       // per generation slot: runs that completed it
 };
 
+// An entity's state before a generation's task: its evaluation counter and the
+// PRNG states of its GA block.
+struct PipeKeep {
+	int gen1;                   // the generation + 1; 0: none kept
+	int evals;
+	uint32_t prng[64];
+};
+
 struct PipeArgs {
 	KArgs ka;                   // tables, dockpars, PRNG states, evaluation counters
 	PopBufs bufs[kPipeBufs];    // generation slot k: conf_cur/e_cur = buffer k, conf/e = buffer (k+1) % nbuf
@@ -112,6 +124,7 @@ struct PipeArgs {
 	float* as_stats;            // (pop + 1) * 3
 	float* as_e;                // runs * pop
 	uint16_t* as_m;             // runs * pop
+	PipeKeep* as_keep;          // nbuf * runs * pop: by generation slot and entity
 	unsigned long long as_min_evals;
 	unsigned int as_frequency;
 	int group_bytes;            // shared memory per pose group (header + scratch)
@@ -272,6 +285,12 @@ __device__ void pipe_worker(const PipeArgs& p)
 			PopBufs pb = p.bufs[g & (p.nbuf - 1)];
 			pb.gen = g;
 			const uint32_t b = (uint32_t)(run * P + ent);
+			if constexpr (AS) {
+				PipeKeep& keep = p.as_keep[(size_t)(g & (p.nbuf - 1)) * ((size_t)R * P) + b];
+				for (int i = G.rank; i < 64; i += TPP) keep.prng[i] = a.prng[(size_t)b * 64 + i];
+				if (G.rank == 0) { keep.gen1 = g + 1; keep.evals = a.evals_new[b]; }
+				G.sync();
+			}
 			pipe_ga<TPP, GA_TPP, SUMS>(a, pb, b, G, S);
 			// num_of_lsentities == pop_size: local-search block b is entity b
 			if constexpr (LSMET == LS_SW) sw_block<TPP, SUMS, true>(a, pb, b, G, S);
@@ -478,6 +497,19 @@ __global__ void __launch_bounds__(256) pipe_final_kernel(PipeArgs p, long long* 
 	}
 }
 
+// Puts back what the generations past the stop changed: the states kept ahead
+// of the first of them.  One warp per entity.
+__global__ void __launch_bounds__(256) pipe_restore_kernel(const PipeArgs p)
+{
+	const int G = p.ctl->stop_gen, n = p.runs * p.pop, lane = threadIdx.x & 31;
+	const int b = blockIdx.x * 8 + (threadIdx.x >> 5);
+	if (G < 0 || b >= n) return;
+	const PipeKeep& keep = p.as_keep[(size_t)(G & (p.nbuf - 1)) * n + b];
+	if (keep.gen1 != G + 1) return;
+	for (int i = lane; i < 64; i += 32) p.ka.prng[(size_t)b * 64 + i] = keep.prng[i];
+	if (lane == 0) p.ka.evals_new[b] = keep.evals;
+}
+
 // Initial check and tasks, the persistent launch, the final accounting; the
 // grid is sized from the kernel's occupancy (persistent: every pose group a
 // worker) and capped by the entities a generation offers.
@@ -504,6 +536,10 @@ static adgpu_status launch_pipe_as(PipeArgs p, long long* d_out, cudaStream_t st
 	ADGPU_CUDA_RET(cudaGetLastError(), "pipeline launch");
 	pipe_final_kernel<<<1, 256, 0, st>>>(p, d_out);
 	ADGPU_CUDA_RET(cudaGetLastError(), "pipeline final");
+	if constexpr (AS) {
+		pipe_restore_kernel<<<(p.runs * p.pop + 7) / 8, 256, 0, st>>>(p);
+		ADGPU_CUDA_RET(cudaGetLastError(), "pipeline restore");
+	}
 	return ADGPU_OK;
 }
 
@@ -586,7 +622,8 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 	const size_t o_ctl = o_runs + runs_b, ctl_b = al(sizeof(PipeCtl)) + 256;
 	// AutoStop: state, statistics, the energies below the threshold and their bins
 	const size_t o_as = o_ctl + ctl_b, as_stats_b = al(autostop_stats_floats(P) * 4);
-	const size_t as_b = as.frequency ? al(sizeof(AutoStopState)) + as_stats_b + al(n * 4) + al(n * 2) : 0;
+	const size_t keep_b = al(sizeof(PipeKeep) * n * nbuf);
+	const size_t as_b = as.frequency ? al(sizeof(AutoStopState)) + as_stats_b + al(n * 4) + al(n * 2) + keep_b : 0;
 	const size_t total = o_as + as_b;
 	if (sc.bytes < total) {
 		if (sc.mem) cudaFree(sc.mem);
@@ -637,7 +674,9 @@ adgpu_status dock_pipelined(const KArgs& base, PipeScratch& sc, int lsmet, int t
 		p.as_state = reinterpret_cast<AutoStopState*>(b); b += al(sizeof(AutoStopState));
 		p.as_stats = reinterpret_cast<float*>(b); b += as_stats_b;
 		p.as_e = reinterpret_cast<float*>(b); b += al(n * 4);
-		p.as_m = reinterpret_cast<uint16_t*>(b);
+		p.as_m = reinterpret_cast<uint16_t*>(b); b += al(n * 2);
+		p.as_keep = reinterpret_cast<PipeKeep*>(b);
+		ADGPU_CUDA_RET(cudaMemsetAsync(b, 0, keep_b, st), "kept states");
 		p.as_frequency = as.frequency;
 		p.as_min_evals = as.min_evals;
 		autostop_init(as_init, P, (int)runs, as.stopstd, as.frequency);

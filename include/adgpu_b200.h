@@ -289,6 +289,8 @@ adgpu_status adgpu_dock_resident(int lsmet, uint32_t num_runs, uint64_t max_eval
  * deviation of the best energies below `stopstd`, --stopstd) and the total
  * evaluations exceed `min_as_evals` (the reference's heuristics minimum; 0
  * without heuristics).  *autostopped reports whether it triggered.  The
+ * PRNG states and the per-entity evaluation counters are left as the last
+ * generation run left them, whatever was run ahead of the stop.  The
  * reference copies all energies to the host for each test; here nothing
  * leaves the device until the loop ends. */
 adgpu_status adgpu_dock_resident_autostop(int lsmet, uint32_t num_runs, uint64_t max_evals, uint32_t max_gens,

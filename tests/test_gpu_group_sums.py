@@ -65,14 +65,20 @@ def test_searches_of_small_launches(grid, heavy, tors, flex, entry, monkeypatch)
     ("sw", 5, 16, 4, 0), ("sw", 13, 32, 8, 0), ("adam", 2, 16, 4, 0), ("adam", 21, 16, 4, 0), ("fire", 2, 16, 4, 0)])
 def test_autostop_pipelined_matches_synchronous(grid, search, runs, heavy, tors, flex, monkeypatch):
     """A budget that ends the docking, and a tolerance wide enough for AutoStop
-    to end it where it can."""
-    for nev, stopstd in ((60_000, 0.15), (250_000, 3.0)):
+    to end it.  The random states and the evaluation counters are part of the
+    result: a docking that goes on from them must not depend on what was run
+    ahead of the stop."""
+    pipelines = search in ("ad", "sw") or (search == "adam" and runs > 20)      # (the others: the same loop twice)
+    for nev, stopstd in ((60_000, 0.15), (3_000_000, 3.0)):
         out = []
         for pipeline in (True, False):
             j, lig = job(grid, heavy, tors, flex, runs, monkeypatch, 0, pipeline)
             r = dock.dock(j, lig.initpop, search, nev, autostop=dock.AutoStopParams(2, stopstd, 0))
-            out.append((r.generations, r.autostopped, r.evals_per_run, r.energies.cpu().numpy(), r.conformations.cpu().numpy()))
+            assert dock.last_stats()["pipelined"] == (pipeline and pipelines)
+            out.append((r.generations, r.autostopped, r.evals_per_run, r.energies.cpu().numpy(), r.conformations.cpu().numpy(),
+                        j.prng.cpu().numpy(), j.evals_new.cpu().numpy()))
         assert out[0][:2] == out[1][:2]
+        assert out[0][1] or nev == 60_000
         for a, b in zip(out[0][2:], out[1][2:]):
             np.testing.assert_array_equal(a, b)
 
