@@ -52,7 +52,8 @@ __device__ __forceinline__ PopBufs bufs_of(const KArgs& a) { return PopBufs{a.co
 // worked on for nothing, and the docking ends only when it does.  So at the end
 // of every eighth iteration (every 32nd with several warps per pose, where a
 // poll is part of the chain of an evaluation) thread 0 reads the stop, its
-// answer goes through S.misc, and the whole group leaves.  B200, dockings of
+// answer goes through S.misc, and the whole group leaves; its evaluations so
+// far are counted (adgpu_dock_stats.evals_executed).  B200, dockings of
 // 100 runs: Solis-Wets 82.4 -> 79.1 ms (7 generations), ADADELTA 122.9 ->
 // 120.7 (30), 50 runs of ADAM with flexible residues 73.7 -> 70.6 (4).
 // POLL: a search of the pipelined loop (in the others the code alone cost a
@@ -228,7 +229,10 @@ __device__ void gradient_ls_block(const KArgs& a, const PopBufs& pb, uint32_t b,
 			if (energy < best_e) best_e = energy;
 		}
 		G.sync();
-		if (abandoned<TPP, POLL>(a, pb, it, G, S.misc)) return;
+		if (abandoned<TPP, POLL>(a, pb, it, G, S.misc)) {
+			if (G.rank == 0) a.evals_new[idx] += (int)it;
+			return;
+		}
 	} while (it < a.dp.max_num_of_iters && (METHOD == LS_ADAM || rho > 0.01f));
 	float* dst = pb.conf + idx * kGenotypeStride;
 	for (int k = G.rank; k < NG; k += TPP) {
@@ -305,7 +309,10 @@ __device__ void fire_block(const KArgs& a, const PopBufs& pb, uint32_t b, const 
 			for (int k = G.rank; k < NG; k += TPP) best[k] = gen[k];
 		}
 		G.sync();
-		if (abandoned<TPP, POLL>(a, pb, it, G, S.misc)) return;
+		if (abandoned<TPP, POLL>(a, pb, it, G, S.misc)) {
+			if (G.rank == 0) a.evals_new[idx] += (int)it;
+			return;
+		}
 	} while (it < a.dp.max_num_of_iters && dt > DT_MIN);
 	float* dst = pb.conf + idx * kGenotypeStride;
 	for (int k = G.rank; k < NG; k += TPP) {
@@ -378,7 +385,10 @@ __device__ void sw_block(const KArgs& a, const PopBufs& pb, uint32_t b, const GT
 		if (succ >= (int)a.dp.cons_limit) { rho *= 2.0f; succ = 0; }
 		else if (fail >= (int)a.dp.cons_limit) { rho *= 0.5f; fail = 0; }
 		G.sync();
-		if (abandoned<TPP, POLL>(a, pb, (uint32_t)iters, G, S.misc)) return;
+		if (abandoned<TPP, POLL>(a, pb, (uint32_t)iters, G, S.misc)) {
+			if (G.rank == 0) a.evals_new[idx] += evals;
+			return;
+		}
 	}
 	float* dst = pb.conf + idx * kGenotypeStride;
 	for (int k = gs + G.rank; k < NG; k += TPP) {

@@ -96,3 +96,20 @@ def test_128_threads_match_host_loop(grid, heavy, tors, flex, monkeypatch):
         assert out[0][0] == out[1][0]
         for a, b in zip(out[0][1:], out[1][1:]):
             np.testing.assert_array_equal(a, b)
+
+
+def test_discarded_evaluations_are_counted(grid, monkeypatch):
+    """evals_executed holds every evaluation executed, those of searches that
+    end early because their generation is discarded among them.  Kept ADAM
+    searches make 300, discarded ones at least the 32 to the first look at the
+    stop."""
+    runs = 3
+    j, lig = job(grid, 32, 8, 0, runs, monkeypatch, 128)
+    r = dock.dock(j, lig.initpop, "adam", nev=200_000)
+    st = dock.last_stats()
+    new = j.evals_new.cpu().numpy()[:runs * lig.dockpars.pop_size]
+    early = new[new < 300]
+    assert st["generations_discarded"] >= 1 and len(early) > 0
+    assert early.min() >= 32
+    kept = r.evals_per_run.sum() - runs * lig.dockpars.pop_size
+    assert st["evals_executed"] >= kept + early.sum()
