@@ -235,10 +235,15 @@ static int auto_tpp(uint32_t n, int kind)
 	return (long)n * 2 <= groups32 ? 64 : 32;
 }
 
-// Pose groups of 128 threads per SM up to which they beat twice as many of 64
-// (33-atom-ligand host loop, ADADELTA, 8 generations, B200: one run 8.5 -> 7.2
-// ms, three 10.0 -> 8.4; at five a group more runs as many rounds as 64's).
-constexpr long kShareGroupsPerSm = 4;
+// Pose groups of 128 threads per SM up to which they beat twice as many of 64:
+// as many as are resident at once.  (Host loop, 4 generations of 150-entity
+// runs, B200, 64 threads and 128, ligands of 16, 36 and 50 atoms: four runs
+// (600 blocks), ADADELTA 4.37 and 3.97, 4.46 and 3.97, 6.34 and 5.20 ms, ADAM
+// 4.95 and 4.65, 7.13 and 6.43, 10.9 and 9.6, FIRE 6.29 and 6.11, 8.32 and 7.94,
+// 12.1 and 11.0; five (750), ADAM 5.04 and 7.50, 7.26 and 9.96, 11.3 and 13.9,
+// FIRE 6.37 and 10.2, 8.43 and 12.9, 12.3 and 17.0, a second round; gradients of
+// 300 poses 23.5 and 22.5 us, of 1,200 25.9 and 28.2.)
+constexpr long kShareGroupsPerSm = ADGPU_MIN_CTAS_GRAD;
 
 template <int KIND>
 adgpu_status launch_kind(const KArgs& a, float* grads, cudaStream_t stream, int tpp)

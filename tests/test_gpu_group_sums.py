@@ -34,11 +34,11 @@ def job(grid, heavy, tors, flex, runs, monkeypatch, tpp=0, pipeline=True):
 
 
 @pytest.mark.parametrize("heavy,tors,flex", LIGANDS)
-@pytest.mark.parametrize("n", [1, 150, 592, 593])
+@pytest.mark.parametrize("n", [1, 150, 592, 593, 740, 741])
 def test_scores_of_small_launches(grid, heavy, tors, flex, n, monkeypatch):
     out = []
     for tpp in (0, 64):
-        _, lig = job(grid, heavy, tors, flex, 4, monkeypatch, tpp)
+        _, lig = job(grid, heavy, tors, flex, 5, monkeypatch, tpp)
         g = lig.initpop[:n].copy()
         g[:, :3] = 20.0 + 0.3 * (g[:, :3] - 20.0)
         out.append(device.score(g, True))
