@@ -324,13 +324,16 @@ adgpu_status dock_resident(ApiState& s, int lsmet, uint32_t runs, uint64_t max_e
 		ADGPU_CUDA(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev), "sm count");
 	}
 	const long tasks = (long)runs * dp.pop_size;
-	// ADAM and FIRE run a fixed number of iterations: entities that all run at
-	// once end together, so with AutoStop there is nothing to work ahead of.
-	// (36-atom ligand, 39 runs, B200, pipelined against synchronous: ADAM 35.9
-	// and 41.4 ms, FIRE 44.4 and 43.3; 5 runs 9.8 and 9.4, 12.8 and 10.9.)
-	// Ligands with CG-G0 pairs have no pipelined kernels with AutoStop.
-	const bool as_gains = as_frequency == 0 || (!s.tables.dev.cgg0 &&
-	                      (lsmet < 2 || (lsmet == 2 && tasks > 4L * ADGPU_MIN_CTAS_GRAD * g_num_sms)));
+	// With AutoStop the pipelined loop serves Solis-Wets, ADADELTA and ADAM, at
+	// every size: no search of theirs was slower in it from one run to 70, 16 and
+	// 36 atoms, 50,000 and 300,000 evaluations a run (B200, synchronous and
+	// pipelined, 36 atoms, 300,000: Solis-Wets, one run 16.8 and 14.7 ms, 20 runs
+	// 29.8 and 26.9, ADADELTA 30.2 and 26.5, 63.7 and 44.1, ADAM 12.3 and 11.0,
+	// 37.8 and 30.1; 70 runs, 50,000: 18.2 and 17.1, 28.9 and 22.0, 28.4 and 26.3;
+	// the graph's capture and the polls cost the synchronous loop 1 to 4 ms).
+	// FIRE's searches end together, and 70 runs took it 34.0 and 35.1 ms: it and
+	// ligands with CG-G0 pairs have no pipelined kernels with AutoStop.
+	const bool as_gains = as_frequency == 0 || (lsmet != 3 && !s.tables.dev.cgg0);
 	if (s.pipeline && as_fits && as_gains && pipeline_applies(dp, runs)) {
 		*autostopped = 0;
 		KArgs base = make_args(s);
@@ -345,12 +348,13 @@ adgpu_status dock_resident(ApiState& s, int lsmet, uint32_t runs, uint64_t max_e
 			as.ga_tpp = tpp ? tpp : auto_tpp(runs * (uint32_t)dp.pop_size, 0);
 			if (tpp == 0) {
 				tpp = auto_tpp(runs * dp.num_of_lsentities, lsmet + 1);
-				// 128 threads with the sums of 64, up to five entities a group,
-				// with ADADELTA (36-atom ligand, B200, against 64 threads: 20
-				// runs 30.0 and 33.8 ms, 25 runs 35.1 and 36.5, 30 runs 41.4 and
-				// 39.0).  Solis-Wets' scoring has no gradient to share out (12
-				// runs 13.5 and 12.7 ms).
-				as.share = tpp == 64 && lsmet == 1 && shares_sums(base.L) && tasks <= 5L * ADGPU_MIN_CTAS_GRAD * g_num_sms;
+				// 128 threads with the sums of 64, up to 17 entities for four
+				// groups, with ADADELTA (300,000 evaluations a run, B200, 64
+				// threads and 128: 16 atoms, 19 runs 30.1 and 28.5 ms, 21 runs 30.5
+				// and 31.3, 24 runs 31.2 and 35.0; 36 atoms 48.4 and 42.2, 48.9
+				// and 46.1, 50.8 and 52.2).  Solis-Wets' scoring has no gradient to
+				// share out (12 runs 12.7 and 13.5 ms).
+				as.share = tpp == 64 && lsmet == 1 && shares_sums(base.L) && 4 * tasks <= 17L * ADGPU_MIN_CTAS_GRAD * g_num_sms;
 			}
 		}
 		return dock_pipelined(base, s.pipe, lsmet, tpp, runs, max_evals, max_gens, as, c1, e1, c2, e2,

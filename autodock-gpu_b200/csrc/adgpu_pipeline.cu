@@ -546,7 +546,10 @@ static adgpu_status launch_pipe_as(PipeArgs p, long long* d_out, cudaStream_t st
 template <int TPP, int LSMET, int GA_TPP = TPP, int SUMS = TPP>
 static adgpu_status launch_pipe(const PipeArgs& p, long long* d_out, cudaStream_t st)
 {
-	if (p.as_state) return launch_pipe_as<TPP, LSMET, GA_TPP, true, SUMS, false>(p, d_out, st);
+	if (p.as_state) {
+		if constexpr (LSMET != LS_FIRE) return launch_pipe_as<TPP, LSMET, GA_TPP, true, SUMS, false>(p, d_out, st);
+		else return fail(ADGPU_ERR_ARG, "pipelined AutoStop with FIRE");
+	}
 	if constexpr (TPP == 128 && LSMET == LS_SW)
 		if (!p.ka.L.cgg0 && few_entities(p)) return launch_pipe_as<TPP, LSMET, GA_TPP, false, SUMS, false, kFewCtasSw>(p, d_out, st);
 	if constexpr (GA_TPP == TPP && SUMS == TPP)
