@@ -184,25 +184,30 @@ class ClockSampler:
 # CPU side: the oracle (C restatement of the reference kernels, one pose per
 # host thread) on inputs prepared by the reference's own front end
 # (oracle/_ref), so that neither this repository's library nor its front end
-# is on that path.
+# is on that path.  Where the reference's sources are not there to build, the
+# CPU baseline's inputs come from this package's front end, whose tables are
+# equal, and there is no reference arm.
 # ---------------------------------------------------------------------------
 def _reference_inputs(config_id: int, npts: int, n_heavy: int, n_tors: int, nrun: int, lsmet: str):
     """Writes the seeded synthetic maps and ligand as .fld/.map/.pdbqt files and
-    prepares them with the reference's own front end (oracle/_ref)."""
+    prepares them with the reference's own front end (oracle/_ref), or this
+    package's.  Returns the job, the oracle's tables and whose front end it was."""
     import tempfile
     from adgpu_b200 import synth          # numpy only: no library is loaded
-    from oracle import oraclepy, refpy
+    from oracle import frontjob, oraclepy, refpy
     w = WORKLOAD
     d = tempfile.mkdtemp(prefix=f"adgpu_ref{config_id}_")
     spec = synth.grid_spec(npts, w["types"], seed=12345 + config_id)
     fld = synth.write_maps(spec, synth.make_maps(spec), d)
     lig_path = os.path.join(d, "ligand.pdbqt")
     synth.write_ligand(synth.ligand_for(config_id, 0, n_heavy, n_tors), lig_path)
+    if not refpy.available():
+        job = frontjob.FrontJob(fld, lig_path, nrun, tuple(w["seed"]), w["pop"])
+        return job, oraclepy.tables_from_refjob(job), "this package's front end"
     job = refpy.RefJob(["--ffile", fld, "--lfile", lig_path, "--nrun", str(nrun), "--seed",
                         ",".join(str(s) for s in w["seed"]), "--lsmet", lsmet, "--heuristics", "0", "--autostop", "0",
                         "--nev", str(w["nev"]), "--psize", str(w["pop"])])
-    ht = oraclepy.tables_from_refjob(job)
-    return job, ht
+    return job, oraclepy.tables_from_refjob(job), "the reference's own front end"
 
 
 class OracleDocking:
@@ -253,14 +258,14 @@ def cpu_baseline(lsmet: str, budget_s: float = 12.0):
     evaluations per run)."""
     w = WORKLOAD
     nthreads = os.cpu_count() or 1
-    job, ht = _reference_inputs(w["config_id"], w["npts"], w["n_heavy"], w["n_tors"], w["nrun"], lsmet)
+    job, ht, prepared_by = _reference_inputs(w["config_id"], w["npts"], w["n_heavy"], w["n_tors"], w["nrun"], lsmet)
     od = OracleDocking(job, ht, lsmet, nthreads)
     e0, t0 = od.evals(), time.perf_counter()
     while time.perf_counter() - t0 < budget_s or od.generations < 1:
         od.generation()
     dt = time.perf_counter() - t0
     v = (od.evals() - e0) / dt
-    job1, ht1 = _reference_inputs(1, 40, 16, 4, 10, lsmet)
+    job1, ht1, _ = _reference_inputs(1, 40, 16, 4, 10, lsmet)
     d1 = OracleDocking(job1, ht1, lsmet, nthreads)
     t1 = time.perf_counter()
     d1.run(w["nev"])
@@ -268,7 +273,7 @@ def cpu_baseline(lsmet: str, budget_s: float = 12.0):
     return {"value": v, "unit": UNIT, "cores": nthreads, "kind": "port",
             "sample": f"{od.generations} complete generations (GA + {lsmet} local search + eval sums, 100 runs x 150) "
                       f"of the workload's docking from its initial population ({od.evals() - e0} evals, {dt:.1f} s), "
-                      f"inputs prepared by the reference's own front end, on {nthreads} host threads",
+                      f"inputs prepared by {prepared_by}, on {nthreads} host threads",
             "cfg1_full_docking": {"workload": "40^3 maps, 16 heavy atoms / 4 torsions, nrun 10, pop 150, nev 2.5M, "
                                               f"lsmet {lsmet}", "seconds": s1, "generations": d1.generations,
                                   "evals_per_s": d1.evals() / s1, "ligands_per_hour": 3600.0 / s1}}
@@ -282,9 +287,13 @@ def run_reference(args, rank, world):
     previous step; value = evaluations / second over the timed steps."""
     if rank != 0:
         return None
+    from oracle import refpy
+    if not refpy.available():
+        return {"impl": "reference", "unavailable": "the reference's sources are not present, so its front end and "
+                                                    "kernels (oracle/_ref) cannot be built"}
     w = WORKLOAD
     nthreads = os.cpu_count() or 1
-    job, ht = _reference_inputs(w["config_id"], w["npts"], w["n_heavy"], w["n_tors"], w["nrun"], args.lsmet)
+    job, ht, _ = _reference_inputs(w["config_id"], w["npts"], w["n_heavy"], w["n_tors"], w["nrun"], args.lsmet)
     od = OracleDocking(job, ht, args.lsmet, nthreads)
     for _ in range(args.warmup):
         od.generation()
@@ -820,8 +829,8 @@ def run_result(args):
     workload (60^3 maps, 40 heavy atoms / 10 torsions, nrun 100, pop 150) on
     the device (adgpu_process_result: population ordering, re-scoring, RMSD,
     clustering; host outputs included) against the reference's own
-    process_result on one host core (oracle/_ref, files switched off), on the
-    same final population."""
+    process_result on one host core (oracle/_ref, files switched off; left out
+    where it is not built), on the same final population."""
     import tempfile
     import torch
     from adgpu_b200 import device, dock, frontend, result, synth
@@ -833,8 +842,10 @@ def run_result(args):
     lig_path = os.path.join(d, "ligand.pdbqt")
     synth.write_ligand(synth.ligand_for(w["config_id"], 0, w["n_heavy"], w["n_tors"]), lig_path)
     seeds = ",".join(str(s) for s in w["seed"])
-    ref = refpy.RefJob(["--ffile", fld, "--lfile", lig_path, "--nrun", str(w["nrun"]), "--seed", seeds,
-                        "--heuristics", "0", "--autostop", "0", "--psize", str(w["pop"])])
+    ref = None
+    if refpy.available():
+        ref = refpy.RefJob(["--ffile", fld, "--lfile", lig_path, "--nrun", str(w["nrun"]), "--seed", seeds,
+                            "--heuristics", "0", "--autostop", "0", "--psize", str(w["pop"])])
     grid = frontend.Grid.read(fld)
     lig = frontend.Ligand(grid, open(lig_path).read(), None, run=frontend.default_dockpars(grid.spacing, w["pop"]),
                           seed=w["seed"], num_runs=w["nrun"])
@@ -859,6 +870,14 @@ def run_result(args):
 
     t_best, out, c_sorted, e_sorted = gpu_time(False)
     t_all, out_all, _, _ = gpu_time(True)
+    line = {"mode": "result", "metric": "ligands/s (result processing)", "workload":
+            f"one docked ligand ({w['n_heavy']} heavy atoms / {w['n_tors']} torsions, {lig.dockpars.num_of_atoms} "
+            f"atoms, {lig.dockpars.num_of_intraE_contributors} pairs), nrun {R}, pop {w['pop']}, {args.lsmet} "
+            f"docking at nev {args.nev}",
+            "gpu_ms_best_entities": 1e3 * t_best, "gpu_ms_all_entities": 1e3 * t_all,
+            "reference_host_ms": None, "speedup_vs_reference": None, "clusters": len(out.clusters), "parity": None}
+    if ref is None:
+        return line
     hp, he = pops0.cpu().numpy(), en0.cpu().numpy()
     tr, reps = [], 0
     t_start = time.perf_counter()
@@ -875,14 +894,8 @@ def run_result(args):
                         for a, b in zip(out.runs, rruns))
     exact = float(np.mean(np.concatenate([(got == want).ravel(), (out.best_xyz == rxyz).ravel(),
                                           (out.peratom == rper).ravel()])))
-    return {"mode": "result", "metric": "ligands/s (result processing)", "workload":
-            f"one docked ligand ({w['n_heavy']} heavy atoms / {w['n_tors']} torsions, {lig.dockpars.num_of_atoms} "
-            f"atoms, {lig.dockpars.num_of_intraE_contributors} pairs), nrun {R}, pop {w['pop']}, {args.lsmet} "
-            f"docking at nev {args.nev}",
-            "gpu_ms_best_entities": 1e3 * t_best, "gpu_ms_all_entities": 1e3 * t_all,
-            "reference_host_ms": 1e3 * t_ref, "reference_reps": reps, "reference_cores": 1,
-            "speedup_vs_reference": t_ref / t_all,
-            "clusters": len(out.clusters), "parity": {
+    return {**line, "reference_host_ms": 1e3 * t_ref, "reference_reps": reps, "reference_cores": 1,
+            "speedup_vs_reference": t_ref / t_all, "parity": {
                 "population_order_identical": bool(np.array_equal(c_sorted.cpu().numpy(), rp) and
                                                    np.array_equal(e_sorted.cpu().numpy(), re_, equal_nan=True)),
                 "clusters_identical": bool(same_clusters),

@@ -1,13 +1,15 @@
 """Shared test helpers: seeded synthetic inputs prepared by the reference's own
-front end (oracle/_ref), and tolerance checks used by the parity tests."""
+front end (oracle/_ref; where that is not built, by this package's, whose
+tables are equal), and tolerance checks used by the parity tests."""
 from __future__ import annotations
 
 import os
 
 import numpy as np
+import pytest
 
 from adgpu_b200 import abi, synth
-from oracle import oraclepy, refpy
+from oracle import frontjob, oraclepy, refpy
 
 SEEDS = "305419896,2271560481,3735928559"
 
@@ -15,7 +17,7 @@ SEEDS = "305419896,2271560481,3735928559"
 class Case:
     """A prepared docking job: reference tables + oracle view of them."""
 
-    def __init__(self, job: refpy.RefJob):
+    def __init__(self, job: refpy.RefJob | frontjob.FrontJob):
         self.job = job
         self.info = job.info
         self.tables = {k: job.blob(k) for k in ("interintra", "intracontrib", "intra", "rotlist", "conform", "grads")}
@@ -56,6 +58,10 @@ def make_case(directory: str, npts: int, map_types, n_heavy: int, n_tors: int, n
                                       anchor=np.array([-3.0 + 6.0 * k, 4.0, 0.0])) for k in range(flexres)]
             synth.write_flexres(res, fr)
         args += ["--flexres", fr]
+    if not refpy.available():
+        if extra_args:
+            pytest.skip("oracle/_ref not built (needs the reference checkout): its front end takes " + str(extra_args[0]))
+        return Case(frontjob.FrontJob(fld, lig, nrun, tuple(int(s) for s in SEEDS.split(",")), pop, fr if flexres else None))
     args += list(extra_args)
     return Case(refpy.RefJob(args))
 
