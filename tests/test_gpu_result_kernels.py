@@ -6,6 +6,8 @@ that does not, and re-scored energies with and without flexible residues.
 The RMSDs and clusters are checked against a plain restatement of
 generate_output's greedy clustering (host/src/processresult.cpp:688-746) on
 the returned poses."""
+import ctypes as C
+import math
 import threading
 
 import numpy as np
@@ -157,3 +159,86 @@ def test_calls_of_several_threads():
     for t in threads:
         t.join()
     assert not errors, errors[0]
+
+
+def pair_sums(xyz, pairs, charges, dp, nlig):
+    """calc_intraE_f (host/src/processligand.cpp:2058-2331) for carbon atoms:
+    intramolecular and ligand-flexres energy, every operation in the host
+    code's type and the float sums in the pairs' order."""
+    m = C.CDLL("libm.so.6")
+    for f in (m.powf, m.expf):
+        f.restype, f.argtypes = C.c_float, [C.c_float] * (2 if f is m.powf else 1)
+    f4, ld = np.float32, np.longdouble
+    dist, r12, r6, elec, desolv = f4(0), [], [], [], []
+    lam, eps0, A, rk = (np.float64(ld(x)) for x in ("0.003627", "78.4", "-8.5525", "7.7839"))
+    B, sigma = eps0 - A, f4(3.6)
+    for _ in range(2048):
+        dist = f4(np.float64(dist) + 0.01)
+        r6.append(f4(1) / f4(m.powf(dist, 6)))
+        r12.append(f4(1) / f4(m.powf(dist, 12)))
+        eps = np.float64(ld(A) + ld(B) / (ld(1) + ld(rk * math.exp(-lam * B * np.float64(dist)))))
+        elec.append(f4(np.float64(f4(dp.coeff_elec)) / (np.float64(dist) * eps)))
+        desolv.append(f4(dp.coeff_desolv) * f4(m.expf(f4(-1) * dist * dist / (f4(2) * sigma * sigma))))
+    eps12 = 0.1662 * math.sqrt(0.150 * 0.150)
+    vA, vB, opt, delta = eps12 * 4.0 ** 12, 2 * eps12 * 4.0 ** 6, f4(4.0), f4(0.5) * f4(dp.smooth)
+    s = [f4(-0.00143 + np.float64(f4(np.float64(f4(dp.qasp)) * abs(q)))) for q in charges]
+    w = f4(33.5103)
+    bin_of = lambda d: max(0, int(np.floor(f4(f4(100) * d) + f4(0.5))) - 1)  # noqa: E731
+    terms = []                                       # (ligand-flexres, vdW, elec, desolv) in the pairs' order
+    for i, j in pairs:
+        d = f4(math.sqrt(((xyz[i] - xyz[j]) ** 2).sum()))
+        vdw = a = b = f4(0)
+        if d < f4(8):
+            sd = d + delta if d <= opt - delta else (opt if d < opt + delta else d - delta)
+            vdw = f4(vA * np.float64(r12[bin_of(sd)])) - f4(vB * np.float64(r6[bin_of(sd)]))
+        if np.float64(d) < 20.48:
+            assert d > f4(dp.elec_min_distance)
+            a = f4(np.float64(f4(charges[i])) * charges[j]) * elec[bin_of(d)]
+            b = (s[i] * w + s[j] * w) * desolv[bin_of(d)]
+        terms.append(((i >= nlig) != (j >= nlig), vdw, a, b))
+
+    def sums(order):
+        vw = el = ds = inter = f4(0)
+        for flex, vdw, a, b in order:
+            if flex:
+                inter = inter + vdw
+                inter = inter + (a + b)
+            else:
+                vw, el, ds = vw + vdw, el + a, ds + b
+        return vw + el + ds, inter
+
+    return sums(terms), sums(terms[::-1])
+
+
+def test_sums_in_the_pairs_order():
+    """The re-scored sums are the host's float sums bit for bit (a ligand and a
+    flexible residue of carbon atoms); in another order they would not be."""
+    runs, pop = 24, 3
+    spec = synth.grid_spec(40, synth.MAP_TYPES_5, seed=77)
+    grid = frontend.Grid.from_maps(synth.quantize_maps(synth.make_maps_fast(spec)), synth.MAP_TYPES_5, spec.spacing, spec.origin)
+
+    def carbon(lines):
+        return [x[:77] + "C" if x.startswith(("ATOM", "HETATM")) else x for x in lines]
+
+    lig_lines = carbon(synth.pdbqt_lines(synth.ligand_for(2, 5, 24, 5))[0])
+    flex_lines = carbon(synth.flexres_text([synth.make_flexres(100, 8, 2, anchor=np.array([-4.0, 3.0, 0.0]))]).splitlines())
+    lig = frontend.Ligand(grid, "\n".join(lig_lines) + "\n", "\n".join(flex_lines) + "\n",
+                          run=frontend.default_dockpars(grid.spacing, pop), num_runs=runs)
+    dp = lig.dockpars
+    charges = [float(x[70:76]) for x in lig_lines + flex_lines if x.startswith(("ATOM", "HETATM"))]
+    assert len(charges) == dp.num_of_atoms > dp.true_ligand_atoms
+    pairs = np.frombuffer(bytes(lig.tables["intracontrib"]), np.uint32)[:2 * dp.num_of_intraE_contributors].reshape(-1, 2).astype(int)
+    pops = torch.from_numpy(lig.initpop.copy()).cuda()
+    en = torch.zeros(runs * pop, device="cuda")
+    out = result.process_result(lig, torch.from_numpy(grid.reference_layout()).cuda(), pops, en, runs)
+    other = 0
+    for r in range(runs):
+        want, reverse = pair_sums(out.best_xyz[r], pairs, charges, dp, dp.true_ligand_atoms)
+        # (of the poses' coordinates, best_xyz's rounding is in the last bit of a double)
+        assert (out.runs[r].intra_e, out.runs[r].interflex_e) == tuple(float(x) for x in want), r
+        other += want != reverse
+    assert other > runs // 2
+    # the ligand's electrostatic map energy from its atoms' own, in their order (atoms outside the box add none)
+    for r in range(runs):
+        e = out.peratom[r, :dp.true_ligand_atoms, 1]
+        assert out.runs[r].inter_e_elec == np.cumsum(np.where(e == 100000.0, np.float32(0), e), dtype=np.float32)[-1], r
