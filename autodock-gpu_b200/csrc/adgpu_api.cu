@@ -19,7 +19,7 @@
 #endif
 // The gradient local searches (ADADELTA, ADAM, FIRE) need more registers than
 // 80 for their scorer without spills; the SM's throughput is the same with 5
-// CTAs as with 6 (the scorer is issue bound).
+// CTAs as with 6 (the L1 data pipe and instruction issue bound the scorer).
 #ifndef ADGPU_MIN_CTAS_GRAD
 #define ADGPU_MIN_CTAS_GRAD 5
 #endif
@@ -274,7 +274,7 @@ struct ApiState {
 	LigandTables tables;       // host-repacked + device copy
 	int tpp = 0;               // threads per pose; 0: chosen per launch (auto_tpp)
 	unsigned int* counters = nullptr;   // library-owned work counters of the local-search launches
-	bool pipeline = true;      // adgpu_dock_resident without AutoStop runs the pipelined loop where it applies
+	bool pipeline = true;      // adgpu_dock_resident[_autostop] run the pipelined loop where it applies
 	PipeScratch pipe;          // its scratch, kept between calls
 	std::mutex mu;
 };
@@ -316,8 +316,9 @@ adgpu_status dock_resident(ApiState& s, int lsmet, uint32_t runs, uint64_t max_e
 {
 	const adgpu_dockpars& dp = s.data.dockpars;
 	memset(&s.pipe.stats, 0, sizeof(s.pipe.stats));
-	// (an AutoStop test sums all energies in one thread: with many of them it
-	// would outlast the pipelined loop's idle limit)
+	// (an AutoStop test adds up all energies in order in one thread, and each
+	// bin's in another: with many of them it would outlast the pipelined loop's
+	// idle limit)
 	const bool as_fits = as_frequency == 0 || (uint64_t)runs * (uint64_t)dp.pop_size <= (1u << 18);
 	if (g_num_sms == 0) {
 		int dev; ADGPU_CUDA(cudaGetDevice(&dev), "device");

@@ -14,9 +14,9 @@
 // rounding of its host build: float operations where its operands are float,
 // double where a double literal promotes them, no fused multiply-adds
 // (explicitly rounded intrinsics).  Which energies fall below the threshold,
-// and into which bin, is found by the whole block in parallel; the float sums
-// that depend on order are then taken by one thread in the reference's order
-// (runs, then entities).
+// and into which bin, is found by the whole group in parallel; the float sums
+// that depend on order are then taken in the reference's order (runs, then
+// entities), the sum over all energies by one thread and each bin's by another.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>

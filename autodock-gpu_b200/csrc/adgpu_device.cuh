@@ -407,8 +407,9 @@ __device__ __forceinline__ GenRot genrot_from(const float* g, bool has_ligand, c
 }
 
 // ---- intramolecular pairs, two per thread with packed FP32 -------------------------
-// sm_100 executes FADD2/FMUL2/FFMA2: one instruction on two floats.  The pair
-// loop is issue bound, so each thread takes two pairs per step and runs their
+// sm_100 executes FADD2/FMUL2/FFMA2: one instruction on two floats.  Each
+// instruction of the pair loop counts (with the L1 data pipe's wavefronts it
+// bounds the scorer), so each thread takes two pairs per step and runs their
 // arithmetic packed; compares, reciprocals and the fixed-point atomics stay
 // per pair.
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
@@ -732,20 +733,22 @@ __host__ __device__ inline bool shares_sums(const LigDev& L)
 // electrostatic, desolvation and CG-G0 energies, and the number of atoms
 // outside the grid.
 //
-// What bounds it.  With 32 threads per pose the GPU is full and instructions
-// count (3,690 warp instructions an evaluation of the 45-atom ligand, half of
-// them the pair loop's).  Groups of 64 and 128 threads serve dockings of few
-// runs, where the chain of one evaluation counts: 7,700 cycles at 128 threads
-// and 38 atoms, of which 1,530 were the orientation genes on one warp, 1,600
-// the pose and intermolecular terms, 890 the sines and cosines.  So the three
-// orientation genes, whose formulas differ, go to different warps (64 threads:
-// host loop of 20 runs 37.5 -> 36.2 ms), and with 128 threads the atom tables
-// are loaded ahead of the sines and cosines, and with up to 64 atoms the upper
-// two warps take the intermolecular terms while the lower two, which built
-// the pose, start on the pairs (a docking of one run 24.4 -> 21.0 ms; the
-// early loads lost 2 % at 64 threads and 32; without gradients the extra
-// barrier cost more than the terms, a Solis-Wets docking of three runs 10.7 ->
-// 11.4 ms).  Every float is computed by the same operations in the same
+// What bounds it.  With 32 threads per pose the GPU is full, and the L1/shared
+// data pipe (1,143 wavefronts an evaluation of the 45-atom ligand's ADADELTA
+// search, 76 % busy) and instruction issue (3,802 warp instructions, 69 %) count
+// together.  Groups of 64 and 128 threads serve dockings of few runs, where the
+// chain of one evaluation counts: some 4,900 cycles at 128 threads and 32 atoms.
+// Before the following it was 7,700 with 38 atoms, of which 1,530 were the
+// orientation genes on one warp, 1,600 the pose and intermolecular terms, 890
+// the sines and cosines.  So the three orientation genes, whose formulas
+// differ, go to different warps (64 threads: docking of 50 27-atom runs with
+// ADAM 27.1 -> 26.5 ms, launches of 150 71-atom entities 12.7 -> 12.5), and
+// with 128 threads the atom tables are loaded ahead of the sines and cosines,
+// and with up to 64 atoms the upper two warps take the intermolecular terms
+// while the lower two, which built the pose, start on the pairs (a docking of
+// one run 24.4 -> 21.0 ms; the early loads lost 2 % at 64 threads and 32;
+// without gradients the extra barrier cost more than the terms, a Solis-Wets
+// docking of three runs 10.7 -> 11.4 ms).  Every float is computed by the same operations in the same
 // order whatever the group does in parallel, and each thread adds up the same
 // terms: results do not depend on it.
 //

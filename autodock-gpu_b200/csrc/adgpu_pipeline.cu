@@ -48,9 +48,10 @@
 // AutoStop leaves the PRNG states and the evaluation counters of its last
 // generation too: each task first keeps its entity's (PipeKeep), and the ones
 // that discarded generations changed are put back.  The synchronous
-// loop ends each generation with its longest searches running alone (36-atom
-// ligand, 20 runs, ADADELTA, 64 threads per pose, B200: 90.3 ms a docking; this
-// loop with the same scorer 75.1 ms, the same final populations).
+// loop ends each generation with its longest searches running alone (20 runs of
+// a 36-atom ligand, 300,000 evaluations a run, ADADELTA, B200: 63.7 ms a
+// docking; this loop 49.5 with 64 threads per pose too, 44.1 with 128 and the
+// sums of 64; the same final populations).
 #include <cuda_runtime.h>
 #include <cstdlib>
 #include <cstring>
@@ -63,7 +64,7 @@
 
 // CTAs per SM the persistent kernel is compiled for.  Gradient local
 // searches: 5 CTAs of 4 pose groups; with 6 the SM's throughput is the same
-// (the scorer is issue bound), but the cfg2 ADADELTA docking's 100 runs x
+// (the L1 data pipe and issue bound the scorer), but the cfg2 ADADELTA docking's 100 runs x
 // 150 entities then leave runs waiting for the stop test (pose groups 95 %
 // busy against 99 %, 158 against 165 M evaluations/s on B200).  Solis-Wets
 // scores energies only, in fewer registers, and gains from the extra warps.
