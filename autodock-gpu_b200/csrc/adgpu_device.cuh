@@ -228,12 +228,11 @@ __device__ __forceinline__ void map_angle(float& a)
 // TPP threads scoring one pose.  TPP == 32 is warp-synchronous; larger groups
 // sync with a named barrier (id 1 + group index within the CTA).
 // CGG0: it scores ligands with CG-G0 pairs (flexible rings).  These have
-// kernels of their own, since a second pair loop beside the first one cost
-// every ligand instruction fetches (with it, without it and at the start of
-// both changes, dockings of 95 runs, B200: ADAM with 22 atoms and 1 torsion
-// 21.4, 20.4 and 20.9 ms, ADADELTA 21.1, 20.0 and 20.3; with 40 atoms and 10
-// torsions 63.4, 63.6 and 68.6 ms, 69.5, 69.2 and 71.9; a branch around the
-// term in the one loop 1.5 % more with 40 atoms).
+// kernels of their own, since a second pair loop beside the first one costs
+// every ligand instruction fetches (dockings of 95 runs, B200, with two loops
+// in a kernel and with one: 22 atoms and 1 torsion, ADAM 21.4 and 20.4 ms,
+// ADADELTA 21.1 and 20.0; 40 atoms and 10 torsions 63.4 and 63.6, 69.5 and
+// 69.2; a branch around the term in one loop for all cost 1.5 % with 40 atoms).
 // AHEAD: the pair loop loads a step's record during the step before, which
 // takes registers.  Groups of 128 threads score few poses per SM, so a step's
 // latency counts.  (With 64 threads it lost 2 to 4 %; without gradients the

@@ -213,7 +213,7 @@ __device__ __forceinline__ void add_row(const float* st, int lane, int nsum, flo
 	}
 }
 
-__host__ __device__ inline size_t rescore_warp_bytes(int N, int NR)
+__host__ __device__ constexpr size_t rescore_warp_bytes(int N, int NR)
 {
 	// coordinates, sines and cosines, per-atom RMSD terms; staged rows
 	return ((size_t)(4 * N + 2 * NR + 8) * sizeof(double) + 15) / 16 * 16 + (size_t)kRows * kRow * sizeof(float);
@@ -841,11 +841,8 @@ adgpu_status process_result_core(const PostLigand& L, const uint32_t* pairs, con
 	else
 		arrange_kernel<float><<<R, 256, (size_t)P * 8, st>>>(populations, energies, (float*)(d + o_scr), P);
 	const int ntask = params->rescore_entities ? R * P : R;
+	static_assert(kWarps * rescore_warp_bytes(ADGPU_MAX_ATOMS, ADGPU_MAX_ROTBONDS) <= 48 * 1024, "no raised limit needed");
 	const size_t wsm = (size_t)kWarps * rescore_warp_bytes(N, NR);
-	if (wsm > 48 * 1024) {
-		e = allow_smem(rescore_kernel, (size_t)kWarps * rescore_warp_bytes(ADGPU_MAX_ATOMS, ADGPU_MAX_ROTBONDS));
-		if (e != cudaSuccess) return done(e, "result smem");
-	}
 	int dev = 0, sms = 148;
 	cudaGetDevice(&dev);
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
